@@ -210,6 +210,10 @@ class NativePlan:
                 raise _lib.FsmError(_lib.FSM_ERR_INVALID, f"linear coefficient with {lc} channels for {C}")
             h = self.shape[-1] // 2 + 1
             half = lin[..., :h].to(device=device, dtype=torch.complex128).contiguous()
+            if lc > 1 and torch.equal(half, half[:, :1].expand_as(half)):
+                # the same symbol for every channel (Laplacian, Biharmonic): one set of tables, a
+                # third of the table reads of a 3D velocity step
+                half, lc = half[:, :1].contiguous(), 1
             self._lin_half = half
             self.lin_batch = lb
             desc.linear_coef = half.data_ptr()
