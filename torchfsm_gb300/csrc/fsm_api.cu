@@ -248,6 +248,9 @@ static int phi_exact(const FsmPlan* p) {
   return bound < 1e-10 ? 1 : 0;
 }
 
+// Steps of one launch of the resident 2D kernel: long runs return to the stream now and then.
+constexpr int32_t kResidentSteps = 2048;
+
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static void free_plan(FsmPlan* p) {
@@ -570,7 +573,10 @@ int fsm_plan_workspace_bytes(const FsmPlan* plan, int32_t batch, int32_t steps, 
 
 int fsm_plan_launch_count(const FsmPlan* plan, int32_t batch, int32_t steps, int64_t* launches) {
   if (!plan || !launches || steps < 0 || batch < 0) return set_error(FSM_ERR_INVALID, "launch_count arguments");
-  if (plan->path == 2 || plan->path == 4) {
+  fsm::ResConfig res;
+  if (fsm::resident_config(plan, batch, &res)) {
+    *launches = steps > 0 ? (steps + kResidentSteps - 1) / kResidentSteps : 1;
+  } else if (plan->path == 2 || plan->path == 4) {
     const int64_t per_stage = (plan->path == 4 ? 4 : 2) +
                               ((plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) ? 1 : 0);
     *launches = (int64_t)fsm::split_parts(plan, batch) * (1 + (int64_t)steps * plan->nstages * per_stage);
@@ -880,10 +886,15 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   // volume passes take them per launch from the host array. The copy reads the caller's host
   // array when it runs, so a captured graph would read it again at every replay: recording is
   // refused while the stream is being captured.
-  if (record_slot && (p->path == 1 || p->path == 3)) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if ((rc = cuda_check(cudaStreamIsCapturing(st, &cs), "stream capture query"))) return rc;
-    if (cs != cudaStreamCaptureStatusNone)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if ((rc = cuda_check(cudaStreamIsCapturing(st, &cap), "stream capture query"))) return rc;
+  // The resident 2D kernel reads the slots from the device too: a captured recording (which the
+  // passes take) stays on the passes.
+  ResConfig res;
+  const bool resident =
+      !prof && !(record_slot && cap != cudaStreamCaptureStatusNone) && resident_config(p, batch, &res);
+  if (record_slot && (p->path == 1 || p->path == 3 || resident)) {
+    if (cap != cudaStreamCaptureStatusNone)
       return set_error(FSM_ERR_INVALID, "integrate: recording is not supported while the stream is being captured");
     if ((rc = cuda_check(cudaMemcpyAsync(d_slots, record_slot, (size_t)(steps + 1) * sizeof(int32_t),
                                          cudaMemcpyHostToDevice, st), "copy record slots")))
@@ -899,11 +910,21 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   if (p->path == 3) return timed(prof, kProfOther, [&] { return launch_pointwise(p, a, st); });
   if (p->path == 1) return timed(prof, kProfOther, [&] { return launch_line(p, a, st); });
 
+  if (resident) {
+    // at most kResidentSteps steps a launch (the next one primes from the state it left)
+    int32_t done = 0;
+    do {
+      a.steps = steps - done < kResidentSteps ? steps - done : kResidentSteps;
+      if ((rc = launch_resident(p, res, a, st))) return rc;
+      done += a.steps;
+      if (a.slots) a.slots += a.steps;
+    } while (done < steps);
+    return FSM_OK;
+  }
+
   // plane (2D) / volume (3D) passes
   float2* arr = (float2*)(ws + off_arrays);
   a.slots = nullptr;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if ((rc = cuda_check(cudaStreamIsCapturing(st, &cap), "stream capture query"))) return rc;
   // Large batches run in parts on streams forked from the caller's: the parts' launches
   // interleave on the device (the column passes of one overlap the row passes of another),
   // which fills the SMs better than one launch sequence of the whole batch.

@@ -126,6 +126,18 @@ int launch_pointwise(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 // Parts (streams) an uncaptured integrate of `batch` samples is split into; 1: one sequence.
 int split_parts(const FsmPlan* p, int batch);
 
+// The shape of a resident 2D launch (fsm_resident.cu): cluster size, kept / other columns and rows
+// per CTA, product pitch, groups per column, threads and shared memory of a CTA.
+struct ResConfig {
+  int cl, ka, kb, pc, fs, rpc, threads;
+  bool tables;
+  size_t smem;
+};
+// Whether a whole integrate of `batch` samples runs in the resident 2D kernel, and in which shape.
+bool resident_config(const FsmPlan* p, int batch, ResConfig* out);
+// a.steps steps of a.B samples in one launch, frames at a.slots (device) when given.
+int launch_resident(const FsmPlan* p, const ResConfig& c, const StepArgs& a, cudaStream_t st);
+
 // Raise a kernel's dynamic shared-memory limit when it needs more than 48 KB. The
 // attribute is per function and per device; the size set is remembered per
 // (kernel, device) so that repeated launches skip the attribute call.

@@ -77,9 +77,18 @@ __device__ __forceinline__ PointK<DIM> point_k(const StepArgs& a, int row, int64
 // reference's state follows. Where a non-last axis sits at its Nyquist index its
 // wavenumber does not change sign under k -> -k, and that Hermitian part is the
 // projection restricted to axes with the same Nyquist status as c.
+// 1 / lap, 1 where lap == 0.
+__device__ __forceinline__ float inv_laplacian(float kx, float ky, float kz, int dim) {
+  float lap = 0.f;
+  lap -= kx * kx;
+  lap -= ky * ky;
+  if (dim == 3) lap -= kz * kz;
+  return (lap == 0.f) ? 1.f : 1.f / lap;
+}
+
 template <int DIM, int CG>
-__device__ __forceinline__ void nv_leray(float2 (&nv)[CG], const PointK<DIM>& pk, int row, int64_t j,
-                                         const StepArgs& a, int nx) {
+__device__ __forceinline__ void nv_leray_il(float2 (&nv)[CG], const PointK<DIM>& pk, int row, int64_t j,
+                                            const StepArgs& a, int nx, float il) {
   const float kk[3] = {pk.kx, pk.ky, pk.kz};
   float sgn[3] = {1.f, 1.f, 1.f};
   int jl, jm = 0;
@@ -94,10 +103,6 @@ __device__ __forceinline__ void nv_leray(float2 (&nv)[CG], const PointK<DIM>& pk
     if (row == nx / 2) sgn[0] = -1.f;
     if (DIM == 3 && jm == a.nm / 2) sgn[1] = -1.f;
   }
-  float lap = 0.f;
-#pragma unroll
-  for (int f = 0; f < CG; ++f) lap -= kk[f] * kk[f];
-  const float il = (lap == 0.f) ? 1.f : 1.f / lap;
   float2 out[CG];
 #pragma unroll
   for (int c = 0; c < CG; ++c) {
@@ -109,6 +114,12 @@ __device__ __forceinline__ void nv_leray(float2 (&nv)[CG], const PointK<DIM>& pk
   }
 #pragma unroll
   for (int c = 0; c < CG; ++c) nv[c] = out[c];
+}
+
+template <int DIM, int CG>
+__device__ __forceinline__ void nv_leray(float2 (&nv)[CG], const PointK<DIM>& pk, int row, int64_t j,
+                                         const StepArgs& a, int nx) {
+  nv_leray_il<DIM, CG>(nv, pk, row, j, a, nx, inv_laplacian(pk.kx, pk.ky, pk.kz, DIM));
 }
 
 // One SETDRK4 stage at one point from its operands already in registers (the recurrences of
