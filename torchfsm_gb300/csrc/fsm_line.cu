@@ -1,7 +1,6 @@
-// Fused 1D integration: one CTA per sample runs every step and stage of the
-// exponential Runge-Kutta scheme with the state, the scheme's running sums
-// and the transform buffer resident in shared memory, and writes recorded
-// frames straight into the trajectory. One launch per integrate call.
+// Fused 1D integration: a group of T threads per sample runs every step and stage of the
+// exponential Runge-Kutta scheme with the state and the scheme's running sums resident in shared
+// memory, and writes recorded frames straight into the trajectory. One launch per integrate call.
 //
 // Nonlinear terms (input dealiased, output not, operator/_base.py:375-403):
 //  FSM_NL_CONVECTION  u u_x: one inverse complex FFT of Z = D + i G with
@@ -9,103 +8,319 @@
 //                     (operator/generic/_convection.py:43-46);
 //  FSM_NL_KS          0.5 u_x^2 (operator/dedicated/_ks_convection.py:27-38).
 // followed by one forward FFT of the real product.
+//
+// Transforms. Thread t keeps the elements t + T j (j < E) in registers from the spectral update
+// through the inverse transform, the product and the forward transform back to the update: the
+// first and the last pass of a transform have radix E, whose inputs and outputs are exactly those
+// elements. Between passes the group exchanges through one of two shared buffers in turn, so an
+// exchange costs one barrier (a buffer is written again only after the other one's barrier). The
+// thread that holds mode k < N/2 updates it and hands the conjugate mode N - k to its owner.
+// Bound: the latency of the chain of passes and exchanges of one sample (a few warps per SM);
+// the transforms ran through shared memory in every pass before, with two barriers each.
+// Measured, us per stage (before -> now): 128 points
+// 1.54 -> 0.57, 256: 2.23 -> 0.76, 1024: 5.3 -> 1.15, 2048: 5.1 -> 1.9, 4096: 10.2 -> 2.9 (1 to 32 samples).
 #include "fsm_internal.cuh"
+#include "fsm_regfft.cuh"
 
 namespace fsm {
 
+// E elements per thread: enough threads for four schedulers where the passes allow it, with first
+// and last radix E (N / E^2 is what the passes between them combine). 128 points take 4 (a full
+// warp: 0.57 us a stage) rather than 8 (half a warp: 0.88). 4096 points take 16 (three passes, 256
+// threads) rather than 8 (four passes, 512 threads): fewer exchanges, fewer instructions.
 template <int N>
 struct LineCfg {
-  static constexpr int G = (N / 16 < 32) ? 32 : N / 16;
-  static constexpr bool BLOCK = G > 32;
+  static constexpr int E = N <= 128 ? 4 : (N <= 2048 ? 8 : 16);
+  static constexpr int T = N / E;
+  static constexpr int G = T < 32 ? 32 : T;  // threads of a sample (lanes beyond T only keep the barriers)
   static constexpr int H = N / 2 + 1;
-  // twiddles, transform buffer, state and the scheme's running sums (at least acc and q)
-  static size_t smem(int n_aux) { return (size_t)(2 * N + (1 + (n_aux > 2 ? n_aux : 2)) * H) * sizeof(float2); }
+  static constexpr int NB = N + N / 16;  // exchange buffer: one word of padding per 16
+  // radix of the pass that follows span P (1: the first one)
+  static constexpr int radix(int P) {
+    const int rem = N / P;
+    if (P == 1 || rem == E) return E;
+    const int mid = rem / E;  // left for the passes before the last
+    return mid >= E ? E : (mid == 16 ? 4 : (mid > 8 ? 8 : mid));
+  }
+  // twiddles of all passes: R x P entries of each pass with span P > 1
+  static constexpr int tw_words() {
+    int w = 0;
+    for (int P = radix(1); P < N; P *= radix(P)) w += radix(P) * P;
+    return w;
+  }
+  static constexpr int TW = tw_words();
+  // a sample's region (float2): two exchange buffers, state and the scheme's running sums
+  __host__ __device__ static constexpr size_t region(int n_aux) {
+    return (size_t)2 * NB + (size_t)(1 + (n_aux > 2 ? n_aux : 2)) * H;
+  }
 };
 
-// Build the inverse-transform input of the stage field `a` at index k.
-template <int N, int KIND>
-__device__ __forceinline__ void line_build(float2* __restrict__ Z, int k, float2 a, float keep, float kxv,
-                                           float scale) {
-  const float2 d = cscale(a, keep * scale);
-  float2 G = make_float2(-kxv * d.y, kxv * d.x);  // i k d
-  const bool selfc = (k == 0) || (k == N / 2);
-  if (KIND == FSM_NL_CONVECTION) {
-    float2 D = d;
-    if (selfc) {
-      D.y = 0.f;
-      G.y = 0.f;
-    }
-    Z[k] = make_float2(D.x - G.y, D.y + G.x);
-    if (!selfc) Z[N - k] = make_float2(D.x + G.y, G.x - D.y);
-  } else {  // FSM_NL_KS
-    if (selfc) G.y = 0.f;
-    Z[k] = G;
-    if (!selfc) Z[N - k] = cconj(G);
+__device__ __forceinline__ int line_pad(int i) { return i + (i >> 4); }
+
+// Twiddles of every pass, [j][k] = W_{R P}^{j k} (consecutive threads read consecutive words).
+template <int N, int P = LineCfg<N>::radix(1)>
+__device__ __forceinline__ void line_twiddles(float2* __restrict__ dst, const float2* __restrict__ master, int tid,
+                                              int nthreads) {
+  if constexpr (P < N) {
+    constexpr int R = LineCfg<N>::radix(P);
+    for (int i = tid; i < R * P; i += nthreads) dst[i] = master[(i / P) * (i % P) * (kTwiddleMax / (R * P))];
+    line_twiddles<N, P * R>(dst + R * P, master, tid, nthreads);
   }
 }
 
-// One sample's integration by G = LineCfg<N>::G threads (t < G): the twiddles `tw` are in shared
-// memory already (visible after the body's first barrier); Z (N), u, acc, q (running sums, n_aux
-// arrays H apart) are the sample's shared-memory region. Every thread of the CTA runs the body the
-// same number of times (its barriers are CTA-wide); `active` false runs it on the data of a valid
-// sample without writing global memory (spare sub-groups of a k_line_multi CTA).
-template <int N, int KIND>
-__device__ __forceinline__ void line_body(const StepArgs& a, int b, int t, const float2* __restrict__ tw,
-                                          float2* __restrict__ Z, float2* __restrict__ u, bool active) {
+// Barrier of the sample's T threads (id: the sample's sub-group in the CTA).
+template <int N>
+__device__ __forceinline__ void line_sync(int id) {
+  if constexpr (LineCfg<N>::T <= 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(LineCfg<N>::T) : "memory");
+}
+
+// The passes of a transform from span P on; v holds the pass's inputs (butterfly b in v[b R ..]).
+template <int N, bool INV, int P>
+__device__ __forceinline__ void line_passes(float2 (&v)[LineCfg<N>::E], float2* __restrict__ cur,
+                                            float2* __restrict__ nxt, const float2* __restrict__ tw, int t, int id,
+                                            bool on) {
   using Cfg = LineCfg<N>;
-  constexpr int H = Cfg::H;
-  constexpr int G = Cfg::G;
+  constexpr int E = Cfg::E, T = Cfg::T, R = Cfg::radix(P), PER = E / R;
+  if (on) {
+#pragma unroll
+    for (int b = 0; b < PER; ++b) {
+      if constexpr (P > 1) {
+        const int k = (t + b * T) & (P - 1);
+#pragma unroll
+        for (int j = 1; j < R; ++j) {
+          float2 w = tw[j * P + k];
+          if (INV) w.y = -w.y;
+          v[b * R + j] = cmul(v[b * R + j], w);
+        }
+      }
+      dft_reg<R, INV>(v + b * R);
+    }
+  }
+  if constexpr (P * R < N) {
+    constexpr int RN = Cfg::radix(P * R), NBN = N / RN;
+    if (on) {
+#pragma unroll
+      for (int b = 0; b < PER; ++b) {
+        const int i = t + b * T, k = i & (P - 1);
+#pragma unroll
+        for (int j = 0; j < R; ++j) cur[line_pad((i - k) * R + k + j * P)] = v[b * R + j];
+      }
+    }
+    line_sync<N>(id);
+    if (on) {
+#pragma unroll
+      for (int b = 0; b < E / RN; ++b)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) v[b * RN + j] = cur[line_pad(t + b * T + j * NBN)];
+    }
+    line_passes<N, INV, P * R>(v, nxt, cur, tw + (P > 1 ? R * P : 0), t, id, on);
+  }
+}
+
+// Exchanges of one transform (which buffer the next exchange takes).
+template <int N>
+constexpr int line_exchanges() {
+  int n = 0;
+  for (int P = LineCfg<N>::radix(1); P < N; P *= LineCfg<N>::radix(P)) ++n;
+  return n;
+}
+
+// The inverse transform's inputs from the stage field `a` at mode k <= N/2: the value at k and, for
+// 0 < k < N/2, the one at N - k.
+template <int N, int KIND>
+__device__ __forceinline__ float2 line_build(int k, float2 a, float mask, float kxv, float2* mirror) {
+  const float2 d = cscale(a, mask);
+  float2 G = make_float2(-kxv * d.y, kxv * d.x);  // i k d
+  const bool selfc = (k == 0) || (k == N / 2);
+  if (selfc) G.y = 0.f;
+  if (KIND == FSM_NL_CONVECTION) {
+    float2 D = d;
+    if (selfc) D.y = 0.f;
+    *mirror = make_float2(D.x + G.y, G.x - D.y);
+    return make_float2(D.x - G.y, D.y + G.x);
+  } else {  // FSM_NL_KS
+    *mirror = cconj(G);
+    return G;
+  }
+}
+
+// One sample's integration by the T threads of its sub-group (`lane_on`; spare lanes of a short
+// sample only keep the barriers or repeat): the twiddles `tw` are in shared memory already (visible after the body's first
+// barrier); `reg` is the sample's shared-memory region. `active` false runs the body on the data of
+// a valid sample without writing global memory (spare sub-groups of a k_line_multi CTA).
+template <int N, int KIND, bool REGS>
+__device__ __forceinline__ void line_body(const StepArgs& a, int b, int t, int id, const float2* __restrict__ tw,
+                                          float2* __restrict__ reg, bool lane_on, bool active) {
+  using Cfg = LineCfg<N>;
+  // with everything in registers the lanes beyond T repeat the work of lane t % T (same values to the
+  // same shared words) instead of branching around it; they write nothing global
+  const bool on = REGS || lane_on;
+  constexpr int H = Cfg::H, T = Cfg::T, E = Cfg::E;
+  constexpr int M = E / 2 + 1;  // modes t + T j, j < M (the last one, N/2, is thread 0's)
+  // the buffers alternate over the exchanges of a stage: two transforms and the conjugate modes
+  constexpr int XF = line_exchanges<N>();
+  float2* u = reg + 2 * Cfg::NB;
   float2* acc = u + H;  // running sums: acc, q (Runge-Kutta: n_aux arrays H apart)
   float2* q = acc + H;
   float2* gstate = a.state + (int64_t)b * H;
-  for (int k = t; k < H; k += G) u[k] = gstate[k];
   const int64_t toff = tab_batch(a, b) * H;
   const float2* tab = a.tab + toff;
   const float2* src = a.src ? a.src + (int64_t)(a.src_batch > 1 ? b : 0) * H : nullptr;
   const int slot0 = a.slots ? a.slots[0] : -1;
-  const bool dc = KIND == FSM_NL_KS && (a.flags & FSM_FLAG_REMOVE_MEAN) && active;
-  if (dc && t == 0) a.dc[(int64_t)a.steps * a.nstages * a.B + b] = u[0];  // initial k = 0 value
-  for (int k = t; k < H; k += G) {
-    if (slot0 >= 0 && active) a.traj[((int64_t)b * a.n_frames + slot0) * H + k] = u[k];
-    if (a.steps > 0) line_build<N, KIND>(Z, k, u[k], (float)a.keepx[k], a.kx[k], a.scale);
-  }
-  __syncthreads();
-  const int ns = a.nstages;
-  for (int step = 0; step < a.steps; ++step) {
-    for (int s = 0; s < ns; ++s) {
-      fft<N, G, Cfg::BLOCK, true>(Z, tw, t);
-      for (int n = t; n < N; n += G) {
-        const float2 z = Z[n];
-        const float p = (KIND == FSM_NL_CONVECTION) ? z.x * z.y : 0.5f * z.x * z.x;
-        Z[n] = make_float2(p, 0.f);
+  const bool dc = KIND == FSM_NL_KS && (a.flags & FSM_FLAG_REMOVE_MEAN) && active && lane_on && t == 0;
+  float2 v[E];
+  float kxr[M], mask[M];
+  // REGS: the state (between stages 0 and 1 exp(dt L / 2) u), the running sums and the tables
+  float2 ru[REGS ? M : 1], racc[REGS ? M : 1], rq[REGS ? M : 1], tE[REGS ? M : 1], tE2[REGS ? M : 1];
+  float tc[4][REGS ? M : 1];  // c1, c4, c5, c6
+  int par = 0;  // the buffer of the next exchange
+
+  // stage field at the thread's modes (registers x) -> inverse transform inputs in v
+  auto emit = [&](const float2 (&x)[M]) {
+    float2* ex = reg + par * Cfg::NB;
+    par ^= 1;
+    if (on) {
+#pragma unroll
+      for (int j = 0; j < M; ++j) {
+        const int k = t + T * j;
+        if (j == M - 1 && t != 0) break;
+        float2 mir;
+        const float2 z = line_build<N, KIND>(k, x[j], mask[j], kxr[j], &mir);
+        if (k > 0 && k < N / 2) ex[line_pad(N - k)] = mir;
+        if (j < M - 1) v[j] = z;
+        else ex[line_pad(k)] = z;
       }
-      __syncthreads();
-      fft<N, G, Cfg::BLOCK, false>(Z, tw, t);
-      const bool last = (s == ns - 1);
-      const bool final_stage = last && (step == a.steps - 1);
-      const int slot = (last && a.slots) ? a.slots[step + 1] : -1;
-      for (int k = t; k < H; k += G) {
-        float2 nv = cscale(Z[k], a.coef);
-        // k = 0 of the product, for the batch-mean fix-up (k_line_dc_fixup)
-        if (dc && k == 0) a.dc[((int64_t)step * ns + s) * a.B + b] = Z[0];
-        if (src) nv = cadd(nv, src[k]);
-        const float2 nxt = etd_stage(a.integ, s, nv, u + k, acc + k, q + k, tab + k, a.ts, H);
-        if (!final_stage) line_build<N, KIND>(Z, k, nxt, (float)a.keepx[k], a.kx[k], a.scale);
-        if (slot >= 0 && active) a.traj[((int64_t)b * a.n_frames + slot) * H + k] = u[k];
+    }
+    line_sync<N>(id);
+    if (on) {
+#pragma unroll
+      for (int j = E / 2; j < E; ++j) v[j] = ex[line_pad(t + T * j)];
+    }
+  };
+
+  float2 x[M];
+  if (on) {
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+      if (j == M - 1 && t != 0) break;
+      const int k = t + T * j;
+      x[j] = gstate[k];
+      kxr[j] = a.kx[k];
+      mask[j] = (float)a.keepx[k] * a.scale;
+      if constexpr (REGS) {
+        ru[j] = x[j];
+        tE[j] = tab[k];
+        tE2[j] = tab[a.ts + k];
+        // the SETDRK coefficients are real (k_phi_tables)
+        tc[0][j] = tab[2 * a.ts + k].x;
+        tc[1][j] = tab[3 * a.ts + k].x;
+        tc[2][j] = tab[4 * a.ts + k].x;
+        tc[3][j] = tab[5 * a.ts + k].x;
+      } else {
+        u[k] = x[j];
       }
-      __syncthreads();
+      if (slot0 >= 0 && active && lane_on) a.traj[((int64_t)b * a.n_frames + slot0) * H + k] = x[j];
     }
   }
-  if (active)
-    for (int k = t; k < H; k += G) gstate[k] = u[k];
+  if (dc) a.dc[(int64_t)a.steps * a.nstages * a.B + b] = x[0];  // initial k = 0 value
+  if (a.steps > 0) emit(x);
+  const int ns = a.nstages;
+#pragma unroll 1
+  for (int step = 0; step < a.steps; ++step) {
+#pragma unroll 1
+    for (int s = 0; s < ns; ++s) {
+      line_passes<N, true, 1>(v, reg + par * Cfg::NB, reg + (par ^ 1) * Cfg::NB, tw, t, id, on);
+      par ^= XF & 1;
+#pragma unroll
+      for (int j = 0; j < E; ++j) {
+        const float p = (KIND == FSM_NL_CONVECTION) ? v[j].x * v[j].y : 0.5f * v[j].x * v[j].x;
+        v[j] = make_float2(p, 0.f);
+      }
+      line_passes<N, false, 1>(v, reg + par * Cfg::NB, reg + (par ^ 1) * Cfg::NB, tw, t, id, on);
+      par ^= XF & 1;
+      const bool last = (s == ns - 1);
+      const int slot = (last && a.slots) ? a.slots[step + 1] : -1;
+      // k = 0 of the product, for the batch-mean fix-up (k_line_dc_fixup)
+      if (dc) a.dc[((int64_t)step * ns + s) * a.B + b] = v[0];
+      if (on) {
+#pragma unroll
+        for (int j = 0; j < M; ++j) {
+          x[j] = cscale(v[j], a.coef);
+          if (src && (j < M - 1 || t == 0)) x[j] = cadd(x[j], src[t + T * j]);
+        }
+        if constexpr (REGS) {
+          // the recurrences of etd_stage_c<FSM_SETDRK4, s>
+#pragma unroll
+          for (int j = 0; j < M; ++j) {
+            const float2 nv = x[j];
+            const float2 c1 = make_float2(tc[0][j], 0.f);
+            if (s == 0) {
+              const float2 e2u = cexpmul(tE2[j], ru[j]);
+              x[j] = cfma(c1, nv, e2u);
+              racc[j] = cfma(make_float2(tc[1][j], 0.f), nv, cexpmul(tE[j], ru[j]));
+              rq[j] = cfma(make_float2(-c1.x, -c1.y), nv, cexpmul(tE2[j], x[j]));
+              ru[j] = e2u;
+            } else if (s == 1) {
+              racc[j] = cfma(make_float2(2.f * tc[2][j], 0.f), nv, racc[j]);
+              x[j] = cfma(c1, nv, ru[j]);
+            } else if (s == 2) {
+              racc[j] = cfma(make_float2(2.f * tc[2][j], 0.f), nv, racc[j]);
+              x[j] = cfma(cscale(c1, 2.f), nv, rq[j]);
+            } else {
+              x[j] = cfma(make_float2(tc[3][j], 0.f), nv, racc[j]);
+              ru[j] = x[j];
+            }
+          }
+        } else {
+          auto stage = [&](auto&& f) {
+#pragma unroll
+            for (int j = 0; j < M; ++j) {
+              if (j == M - 1 && t != 0) break;
+              const int k = t + T * j;
+              x[j] = f(x[j], u + k, acc + k, q + k, tab + k);
+            }
+          };
+          using F2 = float2;
+          if (E > 8 && a.integ == FSM_SETDRK4) {
+            switch (s) {
+              case 0: stage([&](F2 n, F2* pu, F2* pa, F2* pq, const F2* pt) { return etd_stage_c<FSM_SETDRK4, 0>(n, pu, pa, pq, pt, a.ts); }); break;
+              case 1: stage([&](F2 n, F2* pu, F2* pa, F2* pq, const F2* pt) { return etd_stage_c<FSM_SETDRK4, 1>(n, pu, pa, pq, pt, a.ts); }); break;
+              case 2: stage([&](F2 n, F2* pu, F2* pa, F2* pq, const F2* pt) { return etd_stage_c<FSM_SETDRK4, 2>(n, pu, pa, pq, pt, a.ts); }); break;
+              default: stage([&](F2 n, F2* pu, F2* pa, F2* pq, const F2* pt) { return etd_stage_c<FSM_SETDRK4, 3>(n, pu, pa, pq, pt, a.ts); }); break;
+            }
+          } else {
+            stage([&](F2 n, F2* pu, F2* pa, F2* pq, const F2* pt) { return etd_stage(a.integ, s, n, pu, pa, pq, pt, a.ts, H); });
+          }
+        }
+        if (slot >= 0 && active && lane_on) {
+#pragma unroll
+          for (int j = 0; j < M; ++j) {
+            if (j == M - 1 && t != 0) break;
+            const int k = t + T * j;
+            a.traj[((int64_t)b * a.n_frames + slot) * H + k] = x[j];
+          }
+        }
+      }
+      if (!(last && step == a.steps - 1)) emit(x);
+    }
+  }
+  if (lane_on && active) {
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+      if (j == M - 1 && t != 0) break;
+      gstate[t + T * j] = REGS ? ru[REGS ? j : 0] : u[t + T * j];
+    }
+  }
 }
 
-template <int N, int KIND>
+template <int N, int KIND, bool REGS>
 __global__ void __launch_bounds__(LineCfg<N>::G) k_line(StepArgs a) {
+  using Cfg = LineCfg<N>;
   extern __shared__ float2 smem[];
-  float2* tw = smem;
-  load_twiddles(tw, a.tw, kTwiddleMax, N, threadIdx.x, LineCfg<N>::G);
-  line_body<N, KIND>(a, blockIdx.x, threadIdx.x, tw, tw + N, tw + 2 * N, true);
+  line_twiddles<N>(smem, a.tw, threadIdx.x, Cfg::G);
+  __syncthreads();
+  line_body<N, KIND, REGS>(a, blockIdx.x, threadIdx.x % Cfg::T, 0, smem, smem + Cfg::TW, threadIdx.x < Cfg::T, true);
 }
 
 // Serving: the lines of several plans (one per grid size) advanced by one launch. CTAs
@@ -115,35 +330,33 @@ template <int N>
 struct LineMultiCfg {
   static constexpr int G = LineCfg<N>::G;
   static constexpr int P = kLineMultiThreads / G;  // samples per CTA
-  static constexpr int H = N / 2 + 1;
-  __host__ __device__ static size_t region(int n_aux) { return (size_t)N + (size_t)(1 + (n_aux > 2 ? n_aux : 2)) * H; }
-  static size_t smem(int n_aux) { return ((size_t)N + P * region(n_aux)) * sizeof(float2); }
+  static size_t smem(int n_aux) { return (LineCfg<N>::TW + P * LineCfg<N>::region(n_aux)) * sizeof(float2); }
 };
 
-template <int N, int KIND>
+template <int N, int KIND, bool REGS>
 __device__ __forceinline__ void line_multi_cta(const StepArgs& a, int cta) {
   using Cfg = LineMultiCfg<N>;
   extern __shared__ float2 smem[];
-  float2* tw = smem;
-  load_twiddles(tw, a.tw, kTwiddleMax, N, threadIdx.x, kLineMultiThreads);
+  line_twiddles<N>(smem, a.tw, threadIdx.x, kLineMultiThreads);
+  __syncthreads();
   const int sub = threadIdx.x / Cfg::G, t = threadIdx.x % Cfg::G;
   const int b = cta * Cfg::P + sub;
   const bool active = b < a.B;
-  float2* Z = smem + N + (size_t)sub * Cfg::region(a.n_aux);
-  line_body<N, KIND>(a, active ? b : a.B - 1, t, tw, Z, Z + N, active);
+  float2* reg = smem + LineCfg<N>::TW + (size_t)sub * LineCfg<N>::region(a.n_aux);
+  line_body<N, KIND, REGS && LineCfg<N>::E <= 8>(a, active ? b : a.B - 1, t, sub + 1, smem, reg, t < LineCfg<N>::T, active);
 }
 
-template <int KIND>
+template <int KIND, bool REGS>
 __global__ void __launch_bounds__(kLineMultiThreads) k_line_multi(const __grid_constant__ LineMulti m) {
   int j = 0;
   while (j + 1 < m.count && (int)blockIdx.x >= m.cta0[j + 1]) ++j;
   const int cta = (int)blockIdx.x - m.cta0[j];
   switch (m.n[j]) {
-    case 256: line_multi_cta<256, KIND>(m.a[j], cta); break;
-    case 512: line_multi_cta<512, KIND>(m.a[j], cta); break;
-    case 1024: line_multi_cta<1024, KIND>(m.a[j], cta); break;
-    case 2048: line_multi_cta<2048, KIND>(m.a[j], cta); break;
-    case 4096: line_multi_cta<4096, KIND>(m.a[j], cta); break;
+    case 256: line_multi_cta<256, KIND, REGS>(m.a[j], cta); break;
+    case 512: line_multi_cta<512, KIND, REGS>(m.a[j], cta); break;
+    case 1024: line_multi_cta<1024, KIND, REGS>(m.a[j], cta); break;
+    case 2048: line_multi_cta<2048, KIND, REGS>(m.a[j], cta); break;
+    case 4096: line_multi_cta<4096, KIND, REGS>(m.a[j], cta); break;
   }
 }
 
@@ -154,14 +367,23 @@ static void line_multi_shape(int n_aux, int batch, size_t* smem, int* ctas) {
   *ctas = (batch + Cfg::P - 1) / Cfg::P;
 }
 
+template <int N, int KIND, bool REGS>
+static int launch_line_r(const StepArgs& a, cudaStream_t st) {
+  using Cfg = LineCfg<N>;
+  const size_t smem = (Cfg::TW + Cfg::region(a.n_aux)) * sizeof(float2);
+  int rc = prep_smem(k_line<N, KIND, REGS>, smem);
+  if (rc) return rc;
+  k_line<N, KIND, REGS><<<a.B, Cfg::G, smem, st>>>(a);
+  return cuda_check(cudaGetLastError(), "k_line");
+}
+
+// SETDRK4 keeps its state and tables in registers where a thread has few modes (E <= 8).
 template <int N, int KIND>
 static int launch_line_n(const StepArgs& a, cudaStream_t st) {
-  using Cfg = LineCfg<N>;
-  const size_t smem = Cfg::smem(a.n_aux);
-  int rc = prep_smem(k_line<N, KIND>, smem);
-  if (rc) return rc;
-  k_line<N, KIND><<<a.B, Cfg::G, smem, st>>>(a);
-  return cuda_check(cudaGetLastError(), "k_line");
+  if constexpr (LineCfg<N>::E <= 8) {
+    if (a.integ == FSM_SETDRK4) return launch_line_r<N, KIND, true>(a, st);
+  }
+  return launch_line_r<N, KIND, false>(a, st);
 }
 
 template <int KIND>
@@ -228,6 +450,14 @@ __global__ void k_line_dc_fixup(StepArgs a) {
   a.state[(int64_t)b * H] = u;
 }
 
+template <int KIND, bool REGS>
+static int launch_line_multi_k(const LineMulti& m, int total, size_t smem, cudaStream_t st) {
+  int rc = prep_smem(k_line_multi<KIND, REGS>, smem);
+  if (rc) return rc;
+  k_line_multi<KIND, REGS><<<total, kLineMultiThreads, smem, st>>>(m);
+  return cuda_check(cudaGetLastError(), "k_line_multi");
+}
+
 int launch_line_multi(LineMulti& m, int kind, cudaStream_t st) {
   if (m.count < 1 || m.count > kLineMultiMax) return set_error(FSM_ERR_INVALID, "line multi: plan count");
   size_t smem = 0;
@@ -250,17 +480,15 @@ int launch_line_multi(LineMulti& m, int kind, cudaStream_t st) {
     smem = sm > smem ? sm : smem;
   }
   m.cta0[m.count] = total;
-  int rc;
-  if (kind == FSM_NL_KS) {
-    if ((rc = prep_smem(k_line_multi<FSM_NL_KS>, smem))) return rc;
-    k_line_multi<FSM_NL_KS><<<total, kLineMultiThreads, smem, st>>>(m);
-  } else if (kind == FSM_NL_CONVECTION) {
-    if ((rc = prep_smem(k_line_multi<FSM_NL_CONVECTION>, smem))) return rc;
-    k_line_multi<FSM_NL_CONVECTION><<<total, kLineMultiThreads, smem, st>>>(m);
-  } else {
-    return set_error(FSM_ERR_UNSUPPORTED, "line multi: unsupported nonlinear term");
-  }
-  return cuda_check(cudaGetLastError(), "k_line_multi");
+  bool regs = true;
+  for (int j = 0; j < m.count; ++j) regs = regs && m.a[j].integ == FSM_SETDRK4;
+  if (kind == FSM_NL_KS)
+    return regs ? launch_line_multi_k<FSM_NL_KS, true>(m, total, smem, st)
+                : launch_line_multi_k<FSM_NL_KS, false>(m, total, smem, st);
+  if (kind == FSM_NL_CONVECTION)
+    return regs ? launch_line_multi_k<FSM_NL_CONVECTION, true>(m, total, smem, st)
+                : launch_line_multi_k<FSM_NL_CONVECTION, false>(m, total, smem, st);
+  return set_error(FSM_ERR_UNSUPPORTED, "line multi: unsupported nonlinear term");
 }
 
 int launch_line(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
