@@ -417,7 +417,7 @@ int fsm_plan_create(const FsmMeshDesc* mesh, const FsmProgramDesc* prog, double 
   std::vector<uint8_t> tile_zero;
   {
     const int n0 = mesh->n[0];
-    const int w = n0 == 256 ? 16 : (n0 == 128 || n0 == 64) ? 32 : (n0 == 32 || n0 == 16) ? 64 : 0;
+    const int w = n0 == 512 ? 8 : n0 == 256 ? 16 : (n0 == 128 || n0 == 64) ? 32 : (n0 == 32 || n0 == 16) ? 64 : 0;
     if (w && (path == 2 || path == 4)) {
       const int h = mesh->n[nd - 1] / 2 + 1;
       const int64_t inner = p->S / n0;
@@ -436,7 +436,7 @@ int fsm_plan_create(const FsmMeshDesc* mesh, const FsmProgramDesc* prog, double 
   p->hk = p->h;
   if (path == 2) {
     const int n0 = mesh->n[0], n1 = mesh->n[1];
-    const bool reg = is_pow2(n0) && n0 >= 16 && n0 <= 256 && is_pow2(n1) && n1 >= 16 && n1 <= 256;
+    const bool reg = is_pow2(n0) && n0 >= 16 && n0 <= 512 && is_pow2(n1) && n1 >= 16 && n1 <= 512;
     int pre = 0;
     while (pre < p->h && keep[p->koff[1] + pre]) ++pre;
     bool prefix = true;
@@ -446,7 +446,7 @@ int fsm_plan_create(const FsmMeshDesc* mesh, const FsmProgramDesc* prog, double 
   p->wp = p->S / mesh->n[0];
   if (path == 2) {
     const int n0 = mesh->n[0], n1 = mesh->n[1];
-    if (is_pow2(n0) && n0 >= 16 && n0 <= 256 && is_pow2(n1) && n1 >= 16 && n1 <= 256) p->wp = (p->h + 1) & ~1;
+    if (is_pow2(n0) && n0 >= 16 && n0 <= 512 && is_pow2(n1) && n1 >= 16 && n1 <= 512) p->wp = (p->h + 1) & ~1;
   }
   p->ms = (int64_t)mesh->n[0] * p->wp;
   std::vector<float2> tw(kTwiddleMax);
@@ -1024,8 +1024,7 @@ int fsm_rfftn(const FsmPlan* p, int32_t count, const float* in, void* out, void*
     int64_t outer = count;
     for (int j = 0; j < ax; ++j) outer *= p->n[j];
     if (outer > 65535) return set_error(FSM_ERR_UNSUPPORTED, "rfftn: too many fields in one call");
-    rc = transform_c2c_strided_reg(p->n[ax], false, (float2*)out, outer, inner, p->tw, st);
-    if (rc == -1) rc = transform_c2c_strided(p->n[ax], false, (float2*)out, outer, inner, p->tw, st);
+    rc = transform_c2c_strided(p->n[ax], false, (float2*)out, outer, inner, p->tw, st);
     if (rc) return rc;
     inner *= p->n[ax];
   }
@@ -1043,8 +1042,7 @@ int fsm_irfftn(const FsmPlan* p, int32_t count, void* in, float* out, void* stre
     int64_t outer = count;
     for (int j = 0; j < ax; ++j) outer *= p->n[j];
     if (outer > 65535) return set_error(FSM_ERR_UNSUPPORTED, "irfftn: too many fields in one call");
-    rc = transform_c2c_strided_reg(p->n[ax], true, (float2*)in, outer, inner, p->tw, st);
-    if (rc == -1) rc = transform_c2c_strided(p->n[ax], true, (float2*)in, outer, inner, p->tw, st);
+    rc = transform_c2c_strided(p->n[ax], true, (float2*)in, outer, inner, p->tw, st);
     if (rc) return rc;
     inner *= p->n[ax];
   }

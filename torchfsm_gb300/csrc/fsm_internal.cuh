@@ -77,8 +77,6 @@ int integrate_on_workspace(const FsmPlan* p, int32_t batch, void* state, int32_t
 // Recompute the coefficient tables of batch entries [b0, b0 + n) for time step dt (one launch).
 int set_batch_dt_range(FsmPlan* p, int32_t b0, int32_t n, double dt, cudaStream_t st);
 
-int transform_c2c_strided_reg(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw,
-                              cudaStream_t st);  // -1: no register kernel for n
 int launch_volume_axis1_inv(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_volume_axis2(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_volume_axis1_fwd(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
@@ -116,9 +114,7 @@ int launch_plane_row_multi(PlaneMulti& m, int kind, cudaStream_t st);
 // recording, with the pass arrays in `workspace` laid out as fsm_integrate lays them out (fsm_api.cu).
 int plane_args(const FsmPlan* p, void* state, int32_t batch, int32_t steps, void* workspace, size_t workspace_bytes,
                StepArgs* out);
-// Register-FFT plane passes (64..256 points per axis); return -1 when no kernel covers the sizes.
-int launch_plane_col_reg(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
-int launch_plane_row_reg(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
+// The column pass (2D; the x pass of 3D) and the row pass.
 int launch_plane_col(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_plane_row(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_ks_mean(const FsmPlan* p, const StepArgs& a, cudaStream_t st);

@@ -1,5 +1,5 @@
-// Register-FFT versions of the 2D column and row passes (64..256 points per axis): the kernels of
-// one plan and their launchers. The device bodies are in fsm_plane_reg.cuh.
+// The 2D column pass (16..512 points along x; also the 3D x pass, 16..256) and the KS batch mean: the
+// kernels of one plan and their launchers. The device bodies are in fsm_plane_reg.cuh.
 #include "fsm_plane_reg.cuh"
 
 namespace fsm {
@@ -12,11 +12,6 @@ __global__ void __launch_bounds__(256) k_axis0_r(StepArgs a) {
 template <int NX, int KIND, int DIM>
 __global__ void __launch_bounds__(256, 2) k_axis0_r2(StepArgs a) {
   axis0_body<NX, KIND, DIM, true>(a, blockIdx.x, blockIdx.y);
-}
-
-template <int NY, int KIND, int HK>
-__global__ void __launch_bounds__(256, 2) k_plane_row_r(StepArgs a) {
-  plane_row_body<NY, KIND, HK>(a, blockIdx.x, blockIdx.y);
 }
 
 template <int NX, int KIND, int DIM, bool FAST>
@@ -48,29 +43,6 @@ static int launch_axis0_r(const StepArgs& a, cudaStream_t st) {
   return launch_axis0_r_mode<NX, KIND, DIM, false>(a, st);
 }
 
-template <int NY, int KIND, int HK>
-static int launch_row_r_hk(int nx, const StepArgs& a, cudaStream_t st) {
-  using Cfg = RowCfgR<NY>;
-  const int groups_needed = nx / 2;
-  int threads = groups_needed * Cfg::T;
-  if (threads > 256) threads = 256;
-  const int groups = threads / Cfg::T;
-  const size_t smem = (size_t)(NY + groups * Cfg::SCR) * sizeof(float2);
-  int rc = prep_smem(k_plane_row_r<NY, KIND, HK>, smem);
-  if (rc) return rc;
-  dim3 grid(groups_needed / groups, a.B);
-  k_plane_row_r<NY, KIND, HK><<<grid, threads, smem, st>>>(a);
-  return cuda_check(cudaGetLastError(), "k_plane_row_r");
-}
-
-// The 2/3 rule's stored prefix (NY/3 + 1 columns) or every column.
-template <int NY, int KIND>
-static int launch_row_r(int nx, const StepArgs& a, cudaStream_t st) {
-  if (a.hk == NY / 3 + 1) return launch_row_r_hk<NY, KIND, NY / 3 + 1>(nx, a, st);
-  if (a.hk != NY / 2 + 1) return set_error(FSM_ERR_INVALID, "row pass: unexpected stored column count");
-  return launch_row_r_hk<NY, KIND, NY / 2 + 1>(nx, a, st);
-}
-
 template <int KIND, int DIM>
 static int col_r_dispatch(int nx, const StepArgs& a, cudaStream_t st) {
   switch (nx) {
@@ -79,32 +51,20 @@ static int col_r_dispatch(int nx, const StepArgs& a, cudaStream_t st) {
     case 64: return launch_axis0_r<64, KIND, DIM>(a, st);
     case 128: return launch_axis0_r<128, KIND, DIM>(a, st);
     case 256: return launch_axis0_r<256, KIND, DIM>(a, st);
+    case 512:
+      if constexpr (DIM == 2) return launch_axis0_r<512, KIND, DIM>(a, st);
   }
-  return -1;
+  return set_error(FSM_ERR_UNSUPPORTED, "plane pass: unsupported size or nonlinear term");
 }
 
-template <int KIND>
-static int row_r_dispatch(int nx, int ny, const StepArgs& a, cudaStream_t st) {
-  if (nx < 2) return -1;
-  switch (ny) {
-    case 16: return launch_row_r<16, KIND>(nx, a, st);
-    case 32: return launch_row_r<32, KIND>(nx, a, st);
-    case 64: return launch_row_r<64, KIND>(nx, a, st);
-    case 128: return launch_row_r<128, KIND>(nx, a, st);
-    case 256: return launch_row_r<256, KIND>(nx, a, st);
-  }
-  return -1;
-}
-
-// Returns -1 when no register-FFT kernel exists for the sizes (caller falls back).
-int launch_plane_col_reg(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
+int launch_plane_col(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
   if (p->ndim == 3) {
     switch (p->nl) {
       case FSM_NL_CONVECTION: return col_r_dispatch<FSM_NL_CONVECTION, 3>(p->n[0], a, st);
       case FSM_NL_LERAY: return col_r_dispatch<FSM_NL_LERAY, 3>(p->n[0], a, st);
       case FSM_NL_KS: return col_r_dispatch<FSM_NL_KS, 3>(p->n[0], a, st);
     }
-    return -1;
+    return set_error(FSM_ERR_UNSUPPORTED, "plane pass: unsupported size or nonlinear term");
   }
   switch (p->nl) {
     case FSM_NL_VORTICITY: return col_r_dispatch<FSM_NL_VORTICITY, 2>(p->n[0], a, st);
@@ -112,17 +72,31 @@ int launch_plane_col_reg(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
     case FSM_NL_LERAY: return col_r_dispatch<FSM_NL_LERAY, 2>(p->n[0], a, st);
     case FSM_NL_KS: return col_r_dispatch<FSM_NL_KS, 2>(p->n[0], a, st);
   }
-  return -1;
+  return set_error(FSM_ERR_UNSUPPORTED, "plane pass: unsupported size or nonlinear term");
 }
 
-int launch_plane_row_reg(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
-  switch (p->nl) {
-    case FSM_NL_VORTICITY: return row_r_dispatch<FSM_NL_VORTICITY>(p->n[0], p->n[1], a, st);
-    case FSM_NL_CONVECTION:
-    case FSM_NL_LERAY: return row_r_dispatch<FSM_NL_CONVECTION>(p->n[0], p->n[1], a, st);
-    case FSM_NL_KS: return row_r_dispatch<FSM_NL_KS>(p->n[0], p->n[1], a, st);
+// Batch mean of the k = 0 product (KS mean removal): dc = (1/B) sum_b sum_x prod[b][0][x][0..0],
+// the products being transformed along every axis but the first.
+__global__ void k_ks_mean(StepArgs a, int nx) {
+  float acc = 0.f;
+  const int total = a.B * nx;
+  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+    const int b = i / nx, x = i % nx;
+    acc += a.prod[((int64_t)b * a.n_prod) * a.ms + (int64_t)x * a.wp].x;
   }
-  return -1;
+  __shared__ float red[256];
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) a.dc[0] = make_float2(red[0] / (float)a.B, 0.f);
+}
+
+int launch_ks_mean(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
+  k_ks_mean<<<1, 256, 0, st>>>(a, p->n[0]);
+  return cuda_check(cudaGetLastError(), "k_ks_mean");
 }
 
 }  // namespace fsm

@@ -1,8 +1,26 @@
-// Device bodies of the register-FFT 2D column and row passes (64..256 points per axis; the
-// column pass is also the 3D x pass), shared by the kernels of one plan (fsm_plane_reg.cu) and
-// the kernels that advance several plans in one launch (fsm_plane_multi.cu). Same arithmetic
-// and layout as fsm_plane.cu; the transforms run in registers (fsm_regfft.cuh), so each 1D
-// transform touches shared memory once (the pass-1/pass-2 transpose).
+// Device bodies of the register-FFT 2D column and row passes (16..512 points per axis; the column
+// pass is also the 3D x pass), shared by the kernels of one plan (fsm_plane_col.cu,
+// fsm_plane_row.cu), the kernels that advance several plans in one launch (fsm_plane_multi.cu) and,
+// in parts, the resident 2D kernel (fsm_resident.cuh).
+//
+// Each stage of an exponential Runge-Kutta (or Runge-Kutta) scheme on half spectra [B][C][NX][H],
+// H = NY/2 + 1, is two passes over the batch:
+//  column pass (x): forward transform of the products left by the row pass -> N_s (plus the Leray
+//    projection, plus the source); the stage update, recording when a step completes; the next
+//    stage's fields (2/3 mask, 1/(NX NY), x derivatives, streamfunction) and their inverse transform.
+//  row pass (y): c2r of those fields (y derivatives), the product, r2c.
+// Programs (nonlinear term, operator/_base.py:375-403; input masked only):
+//  FSM_NL_VORTICITY  psi = -w/lap (1 at k = 0), u = (d_y psi, -d_x psi),
+//                    product u.grad(w) (operator/dedicated/_navier_stokes.py:40-46)
+//                    mid: psi, i kx psi, w, i kx w
+//  FSM_NL_CONVECTION (u.grad)u with C = 2 (operator/generic/_convection.py:43-46)
+//                    mid: u0, i kx u0, u1, i kx u1; products conv0 + i conv1
+//  FSM_NL_LERAY      convection, then N = i k p - conv, p = (i k . conv)/lap
+//                    (operator/dedicated/_navier_stokes.py:246-254)
+//  FSM_NL_KS         0.5|grad phi|^2, mean over the batch removed on request
+//                    (operator/dedicated/_ks_convection.py:27-38); mid: phi, i kx phi
+// The transforms run in registers (fsm_regfft.cuh), so each 1D transform touches shared memory once
+// (512 points: twice).
 //
 // Row pass: a group of T lanes owns a pair of rows. It loads the mid fields
 // straight from global memory into the transform layout (the Hermitian
@@ -39,7 +57,7 @@ struct ColCfg {
   static constexpr int T = RS::T;
   static constexpr int E = RS::E;
   static constexpr int W = 256 / T;
-  static constexpr int NEED = (NX > E * (T + 1)) ? NX : E * (T + 1);
+  static constexpr int NEED = (NX > reg_scratch<NX>()) ? NX : reg_scratch<NX>();
   static constexpr int P = NEED | 1;  // odd pitch: a row across W columns hits W distinct banks
 };
 

@@ -10,6 +10,9 @@
 // transpose through shared memory (pitch T+1, conflict-free for 8-byte
 // words), then pass 2: E/T radix-T DFTs over t per lane, which leave output
 // K = t + T j' in register j'.
+//
+// 512 = 16 x 2 x 16 over a full warp: three passes and two exchanges (more lanes than elements per
+// lane, so the second radix cannot be the lane count), with the same layout on entry and exit.
 #pragma once
 
 #include "fsm_fft.cuh"
@@ -18,6 +21,10 @@ namespace fsm {
 
 template <int N>
 struct RegShape;
+template <>
+struct RegShape<512> {
+  static constexpr int T = 32, E = 16;
+};
 template <>
 struct RegShape<256> {
   static constexpr int T = 16, E = 16;
@@ -37,11 +44,6 @@ struct RegShape<32> {
 template <>
 struct RegShape<16> {
   static constexpr int T = 4, E = 4;
-};
-
-template <int N>
-struct HasRegShape {
-  static constexpr bool value = (N == 16 || N == 32 || N == 64 || N == 128 || N == 256);
 };
 
 // 16-point DFT as 4 x 4 (inputs v[r + 4 l], outputs X[q + 4 s]).
@@ -94,16 +96,61 @@ template <int N>
 __device__ __forceinline__ void load_reg_twiddles(float2* twt, const float2* __restrict__ master, int tid,
                                                   int nthreads) {
   constexpr int T = RegShape<N>::T, E = RegShape<N>::E;
-  for (int i = tid; i < T * E; i += nthreads) {
-    const int m = i / T, t = i % T;
-    twt[i] = master[(t * m) * (kTwiddleMax / N)];
+  if constexpr (N == 512) {
+    // W_32^k (k < 16), then W_512^{j k} at 16 + 32 (j - 1) + k (1 <= j < 16, k < 32)
+    for (int i = tid; i < 16 + 15 * 32; i += nthreads) {
+      const int r = i - 16;
+      twt[i] = i < 16 ? master[i * (kTwiddleMax / 32)] : master[((r / 32 + 1) * (r % 32)) * (kTwiddleMax / 512)];
+    }
+  } else {
+    for (int i = tid; i < T * E; i += nthreads) {
+      const int m = i / T, t = i % T;
+      twt[i] = master[(t * m) * (kTwiddleMax / N)];
+    }
   }
 }
 
-// Scratch a group needs: E rows of T+1 words.
+// Scratch a group needs: E rows of T+1 words (512: one word of padding per 16).
 template <int N>
 constexpr int reg_scratch() {
-  return RegShape<N>::E * (RegShape<N>::T + 1);
+  return N == 512 ? 512 + 32 : RegShape<N>::E * (RegShape<N>::T + 1);
+}
+
+template <bool INV>
+__device__ __forceinline__ void reg_fft512(float2 (&v)[16], float2* __restrict__ x, const float2* __restrict__ twt,
+                                           int t) {
+  auto pad = [](int i) { return i + (i >> 4); };
+  auto tw = [&](float2 a, float2 w) {
+    if (INV) w.y = -w.y;
+    return cmul(a, w);
+  };
+  dft16<INV>(v);  // elements t + 32 j -> outputs 16 t + j
+#pragma unroll
+  for (int j = 0; j < 16; ++j) x[17 * t + j] = v[j];
+  __syncwarp();
+  const int k2 = t & 15;
+  const float2 w2 = twt[k2];  // every butterfly i = t + 32 b has i mod 16 = t mod 16
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    v[2 * b] = x[pad(t + 32 * b)];
+    v[2 * b + 1] = tw(x[pad(t + 32 * b + 256)], w2);
+    dft2<INV>(v + 2 * b);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const int base = (t + 32 * b - k2) * 2 + k2;
+    x[pad(base)] = v[2 * b];
+    x[pad(base + 16)] = v[2 * b + 1];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    v[j] = x[pad(t + 32 * j)];
+    if (j > 0) v[j] = tw(v[j], twt[16 + 32 * (j - 1) + t]);
+  }
+  dft16<INV>(v);
+  __syncwarp();
 }
 
 // In-register FFT of the group's N points (see file comment). `scratch` holds
@@ -112,6 +159,10 @@ constexpr int reg_scratch() {
 template <int N, bool INV>
 __device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::E], float2* __restrict__ scratch,
                                         const float2* __restrict__ twt, int t) {
+  if constexpr (N == 512) {
+    reg_fft512<INV>(v, scratch, twt, t);
+    return;
+  } else {
   constexpr int T = RegShape<N>::T, E = RegShape<N>::E;
   constexpr int PER = E / T;
   dft_reg<E, INV>(v);
@@ -135,6 +186,7 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::E], float2* __r
     for (int k = 0; k < T; ++k) v[p + PER * k] = w[k];
   }
   __syncwarp();
+  }
 }
 
 }  // namespace fsm

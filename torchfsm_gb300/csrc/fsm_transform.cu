@@ -1,10 +1,6 @@
-// Multi-dimensional real transforms built from two axis kernels:
-//  * r2c / c2r along the contiguous last axis: two real rows travel as one
-//    complex row z = a + i b (forward: split with Hermitian symmetry;
-//    inverse: Z = A + i B over the Hermitian extension of each half spectrum);
-//  * complex-to-complex along a strided outer axis on tiles of 8 adjacent
-//    columns, staged through shared memory so that global accesses stay
-//    coalesced and each warp transforms one column.
+// Real transforms along the contiguous last axis: two real rows travel as one complex row
+// z = a + i b (forward: split with Hermitian symmetry; inverse: Z = A + i B over the Hermitian
+// extension of each half spectrum). The outer axes are k_c2c_strided_r's (fsm_volume.cu).
 // These serve fsm_rfftn / fsm_irfftn (FourierMesh.fft / ifft(...).real,
 // mesh.py:481-491) for the initial spectrum, the returned fields and the
 // recorded trajectories.
@@ -84,32 +80,6 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_c2r_last(const float2* _
   }
 }
 
-// data: [outer][N][inner] complex; transform along the middle axis, in place.
-constexpr int kColW = 8;
-template <int N, bool INV>
-__global__ void __launch_bounds__(256) k_c2c_strided(float2* __restrict__ data, int64_t inner,
-                                                     const float2* __restrict__ master) {
-  constexpr int P = N + 2;  // column pitch (bank-conflict-free transposed writes)
-  extern __shared__ float2 smem[];
-  float2* tw = smem;
-  float2* tile = smem + N;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t c0 = (int64_t)blockIdx.x * kColW;
-  float2* base = data + (int64_t)blockIdx.y * N * inner;
-  load_twiddles(tw, master, kTwiddleMax, N, threadIdx.x, 256);
-  for (int idx = threadIdx.x; idx < N * kColW; idx += 256) {
-    const int row = idx / kColW, col = idx % kColW;
-    if (c0 + col < inner) tile[col * P + row] = base[(int64_t)row * inner + c0 + col];
-  }
-  __syncthreads();
-  if (c0 + w < inner) fft<N, 32, false, INV>(tile + w * P, tw, lane);
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < N * kColW; idx += 256) {
-    const int row = idx / kColW, col = idx % kColW;
-    if (c0 + col < inner) base[(int64_t)row * inner + c0 + col] = tile[col * P + row];
-  }
-}
-
 template <int N>
 static int launch_r2c(const float* in, float2* out, int64_t rows, const float2* tw, cudaStream_t st) {
   using Cfg = RowCfg<N>;
@@ -130,16 +100,6 @@ static int launch_c2r(const float2* in, float* out, int64_t rows, float scale, c
   const int64_t blocks = (pairs + Cfg::GROUPS - 1) / Cfg::GROUPS;
   k_c2r_last<N><<<(unsigned)blocks, Cfg::THREADS, Cfg::SMEM, st>>>(in, out, rows, scale, tw);
   return cuda_check(cudaGetLastError(), "k_c2r_last");
-}
-
-template <int N, bool INV>
-static int launch_c2c(float2* data, int64_t outer, int64_t inner, const float2* tw, cudaStream_t st) {
-  const size_t smem = (size_t)(N + kColW * (N + 2)) * sizeof(float2);
-  int rc = prep_smem(k_c2c_strided<N, INV>, smem);
-  if (rc) return rc;
-  dim3 grid((unsigned)((inner + kColW - 1) / kColW), (unsigned)outer);
-  k_c2c_strided<N, INV><<<grid, 256, smem, st>>>(data, inner, tw);
-  return cuda_check(cudaGetLastError(), "k_c2c_strided");
 }
 
 int transform_r2c_last(int n, const float* in, float2* out, int64_t rows, const float2* tw, cudaStream_t st) {
@@ -171,24 +131,6 @@ int transform_c2r_last(int n, const float2* in, float* out, int64_t rows, float 
     case 4096: return launch_c2r<4096>(in, out, rows, scale, tw, st);
   }
   return set_error(FSM_ERR_UNSUPPORTED, "c2r: unsupported length " + std::to_string(n));
-}
-
-int transform_c2c_strided(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw,
-                          cudaStream_t st) {
-#define FSM_C2C_CASE(NN)                                                                        \
-  case NN:                                                                                      \
-    return inverse ? launch_c2c<NN, true>(data, outer, inner, tw, st)                           \
-                   : launch_c2c<NN, false>(data, outer, inner, tw, st);
-  switch (n) {
-    FSM_C2C_CASE(16)
-    FSM_C2C_CASE(32)
-    FSM_C2C_CASE(64)
-    FSM_C2C_CASE(128)
-    FSM_C2C_CASE(256)
-    FSM_C2C_CASE(512)
-  }
-#undef FSM_C2C_CASE
-  return set_error(FSM_ERR_UNSUPPORTED, "c2c: unsupported length " + std::to_string(n));
 }
 
 // Per-field NaN/Inf flags: one block per field.

@@ -8,7 +8,7 @@
 //     (Convection, operator/generic/_convection.py:43-46), or 0.5 |grad phi|^2
 //     (KSConvection, operator/dedicated/_ks_convection.py:27-38);
 //   axis 1 forward: in-place y transform of the products (k_c2c_strided_r);
-//   axis 0 (k_axis0_r in fsm_plane_reg.cu): x transform, stage update, next fields.
+//   axis 0 (k_axis0_r in fsm_plane_col.cu): x transform, stage update, next fields.
 #include "fsm_internal.cuh"
 #include "fsm_regfft.cuh"
 
@@ -20,7 +20,7 @@ struct TileCfg {
   static constexpr int T = RS::T;
   static constexpr int E = RS::E;
   static constexpr int W = 256 / T;
-  static constexpr int NEED = (N > E * (T + 1)) ? N : E * (T + 1);
+  static constexpr int NEED = (N > reg_scratch<N>()) ? N : reg_scratch<N>();
   static constexpr int P = NEED | 1;
 };
 
@@ -80,7 +80,7 @@ static int launch_c2c_r(float2* data, int64_t outer, int64_t inner, const float2
   return cuda_check(cudaGetLastError(), "k_c2c_strided_r");
 }
 
-int transform_c2c_strided_reg(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw,
+int transform_c2c_strided(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw,
                               cudaStream_t st) {
 #define FSM_C2CR_CASE(NN)                                                                    \
   case NN:                                                                                   \
@@ -92,9 +92,10 @@ int transform_c2c_strided_reg(int n, bool inverse, float2* data, int64_t outer, 
     FSM_C2CR_CASE(64)
     FSM_C2CR_CASE(128)
     FSM_C2CR_CASE(256)
+    FSM_C2CR_CASE(512)
   }
 #undef FSM_C2CR_CASE
-  return -1;
+  return set_error(FSM_ERR_UNSUPPORTED, "c2c: unsupported length " + std::to_string(n));
 }
 
 // ---------------------------------------------------------------------------
@@ -379,9 +380,7 @@ int launch_volume_axis2(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
 }
 
 int launch_volume_axis1_fwd(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
-  const int rc = transform_c2c_strided_reg(p->n[1], false, a.prod, (int64_t)a.B * a.n_prod * p->n[0], a.H, p->tw, st);
-  if (rc == -1) return set_error(FSM_ERR_UNSUPPORTED, "3D: unsupported second-axis length");
-  return rc;
+  return transform_c2c_strided(p->n[1], false, a.prod, (int64_t)a.B * a.n_prod * p->n[0], a.H, p->tw, st);
 }
 
 }  // namespace fsm
