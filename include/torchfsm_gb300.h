@@ -223,6 +223,10 @@ int fsm_nonfinite_flags(const FsmPlan* plan, int32_t count, const void* fields, 
  *   float [points]). */
 int fsm_adj_accumulate(int64_t n, const void* x, const void* y, double* tbar, void* stream);
 
+/* d(table)/dL of the SETDRK4 coefficient tables E, E2, c1, c4, c5, c6 at n real symbol values `linear`
+ * (DEVICE double [n]) for time step dt, into DEVICE double out[6][n]. */
+int fsm_adj_table_derivs(int64_t n, const double* linear, double dt, double* out, void* stream);
+
 /* One step of the discrete adjoint of the plan's SETDRK4 step for a Convection program
  * (integrator/_stable_etdrk/_setdrk_step.py:55-82 with operator/generic/_convection.py:43-46;
  * the reference gets it from torch autograd, operator/_base.py:731-735). The plan must be

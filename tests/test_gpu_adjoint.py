@@ -160,3 +160,22 @@ def test_recomputed_segments_match_reference_autograd(name):
     tol_c = max(1e-4, 2 * float(np.nan_to_num(g["fp32_grad_coef_rel"])))  # NaN: the float32 autograd is NaN
     print(f"{name}: grad u0 rel-L2 {err_u:.2e} (bound {tol_u:.1e}), grad coef rel {err_c:.2e} (bound {tol_c:.1e})")
     assert err_u <= tol_u and err_c <= tol_c
+
+
+def test_table_derivatives_of_the_library_match_the_contour_formulas():
+    """fsm_adj_table_derivs over both of its branches (series for |dt L| < 0.5, closed forms above)
+    and the switch between them, against the contour means in float64."""
+    from torchfsm_gb300 import _lib, adjoint
+
+    dt = 0.01
+    z = torch.cat([torch.tensor([0.0, -1e-9, 1e-6, -0.4999999, -0.5, 0.5, 0.4999999, 3.0]),
+                   -torch.logspace(-6, 3, 400)]).double().cuda()
+    L = (z / dt).contiguous()
+    out = torch.empty((6, L.numel()), dtype=torch.float64, device="cuda")
+    _lib.check(_lib.load().fsm_adj_table_derivs(L.numel(), L.data_ptr(), dt, out.data_ptr(),
+                                                torch.cuda.current_stream().cuda_stream))
+    ref = adjoint._table_derivatives(L.to(torch.complex128), dt, 32, 2.0)
+    for t in range(6):
+        # at |z| = 0.5 the closed forms lose 4/z^4 x 2^-53 x ~10 = 7e-14 of values of order 0.1
+        scale = ref[t].abs().max()
+        assert float((out[t] - ref[t]).abs().max() / scale) < 1e-11, t

@@ -74,6 +74,7 @@ EXPORTS = (
     "fsm_irfftn",
     "fsm_nonfinite_flags",
     "fsm_adj_accumulate",
+    "fsm_adj_table_derivs",
     "fsm_adj_vjp_products",
     "fsm_adj_vjp_combine",
     "fsm_step_adjoint_workspace_bytes",
@@ -170,6 +171,7 @@ def load(path: Optional[str] = None) -> ctypes.CDLL:
         lib.fsm_irfftn.argtypes = [vp, i32, vp, vp, vp]
         lib.fsm_nonfinite_flags.argtypes = [vp, i32, vp, vp, vp]
         lib.fsm_adj_accumulate.argtypes = [i64, vp, vp, vp, vp]
+        lib.fsm_adj_table_derivs.argtypes = [i64, vp, ctypes.c_double, vp, vp]
         lib.fsm_adj_vjp_products.argtypes = [i32, i32, i64, ctypes.c_float, vp, vp, vp, vp, vp, vp, vp, vp]
         lib.fsm_adj_vjp_combine.argtypes = [i32, i32, i64, vp, vp, vp, vp, vp, vp, vp, vp]
         lib.fsm_step_adjoint_workspace_bytes.argtypes = [vp, i32, ctypes.POINTER(sz)]

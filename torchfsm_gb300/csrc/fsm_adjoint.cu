@@ -72,6 +72,63 @@ __global__ void k_adj_vjp_combine(int BC, int64_t S, const float2* __restrict__ 
   }
 }
 
+// d(table)/dL of the six SETDRK4 tables of a real symbol L, in FP64: E' = dt e^z, E2' = dt e^{z/2} / 2,
+// and c' = dt^2 g'(z) for the tables c = dt g(z), z = dt L. Near 0 from the Taylor series of the g (their
+// coefficients come from expanding e^z), elsewhere from the closed forms: g1 = (e^{z/2} - 1) / z, and
+// g = N / z^3 (c4, c5, c6) with g' = (N' z - 3 N) / z^4. Bound: FP64 arithmetic.
+struct DPhiTaylor {
+  double h[24], a[24], b[24], c[24];
+};
+constexpr DPhiTaylor dphi_taylor() {
+  DPhiTaylor t{};
+  double fact = 1.0, half = 0.5;  // k!, 2^-(k+1)
+  for (int k = 0; k < 24; ++k) {
+    const double f1 = fact * (k + 1), f3 = f1 * (k + 2) * (k + 3);
+    t.h[k] = k * half / f1;
+    t.a[k] = (double)k * (k + 1) * (k + 1) / f3;
+    t.b[k] = (double)k * (k + 1) / f3;
+    t.c[k] = (double)k * (1 - k) / f3;
+    fact = f1;
+    half *= 0.5;
+  }
+  return t;
+}
+static __constant__ DPhiTaylor kDPhiTaylor = dphi_taylor();
+
+__global__ void k_adj_table_derivs(int64_t n, const double* __restrict__ L, double dt, double* __restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double z = dt * L[i];
+    const double ez = exp(z), eh = exp(0.5 * z);
+    double g1 = 0.0, g4 = 0.0, g5 = 0.0, g6 = 0.0;
+    if (fabs(z) < 0.5) {
+      double zk = 1.0;  // z^(k-1)
+      for (int k = 1; k < 24; ++k) {
+        g1 += kDPhiTaylor.h[k] * zk;
+        g4 += kDPhiTaylor.a[k] * zk;
+        g5 += kDPhiTaylor.b[k] * zk;
+        g6 += kDPhiTaylor.c[k] * zk;
+        zk *= z;
+      }
+    } else {
+      const double r = 1.0 / z, r2 = r * r, r4 = r2 * r2;
+      const double n4 = -4.0 - z + ez * (4.0 - 3.0 * z + z * z), d4 = -1.0 + ez * (1.0 - z + z * z);
+      const double n5 = 2.0 + z + ez * (z - 2.0), d5 = 1.0 + ez * (z - 1.0);
+      const double n6 = -4.0 - 3.0 * z - z * z + ez * (4.0 - z), d6 = -3.0 - 2.0 * z + ez * (3.0 - z);
+      g1 = (0.5 * z * eh - (eh - 1.0)) * r2;
+      g4 = (d4 * z - 3.0 * n4) * r4;
+      g5 = (d5 * z - 3.0 * n5) * r4;
+      g6 = (d6 * z - 3.0 * n6) * r4;
+    }
+    const double d2 = dt * dt;
+    out[i] = dt * ez;
+    out[n + i] = 0.5 * dt * eh;
+    out[2 * n + i] = d2 * g1;
+    out[3 * n + i] = d2 * g4;
+    out[4 * n + i] = d2 * g5;
+    out[5 * n + i] = d2 * g6;
+  }
+}
+
 inline unsigned grid_for(int64_t n) {
   int64_t g = (n + 255) / 256;
   return (unsigned)(g > 152 * 16 ? 152 * 16 : (g < 1 ? 1 : g));
@@ -389,6 +446,13 @@ int fsm_adj_accumulate(int64_t n, const void* x, const void* y, double* tbar, vo
   if (n == 0) return FSM_OK;
   k_adj_accumulate<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(n, (const float2*)x, (const float2*)y, tbar);
   return cuda_check(cudaGetLastError(), "k_adj_accumulate");
+}
+
+int fsm_adj_table_derivs(int64_t n, const double* linear, double dt, double* out, void* stream) {
+  if (n < 0 || !(dt > 0.0) || (n > 0 && (!linear || !out))) return set_error(FSM_ERR_INVALID, "adj_table_derivs arguments");
+  if (n == 0) return FSM_OK;
+  k_adj_table_derivs<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(n, linear, dt, out);
+  return cuda_check(cudaGetLastError(), "k_adj_table_derivs");
 }
 
 int fsm_adj_vjp_products(int32_t batch, int32_t nd, int64_t points, float scale, const float* nbar, const float* u,
