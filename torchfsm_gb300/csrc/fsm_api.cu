@@ -488,6 +488,15 @@ int fsm_plan_create(const FsmMeshDesc* mesh, const FsmProgramDesc* prog, double 
     for (int j = pre; j < p->h; ++j) prefix = prefix && !keep[p->koff[1] + j];
     if (reg && prefix && pre == n1 / 3 + 1) p->hk = pre;
   }
+  if (path == 4) {
+    // 3D: the stage fields' kept last-axis prefix, when the mask keeps n2/3 + 1 columns
+    const int n2 = mesh->n[2];
+    int pre = 0;
+    while (pre < p->h && keep[p->koff[2] + pre]) ++pre;
+    bool prefix = true;
+    for (int j = pre; j < p->h; ++j) prefix = prefix && !keep[p->koff[2] + j];
+    if (prefix && pre == n2 / 3 + 1) p->hk = pre;
+  }
   p->wp = p->S / mesh->n[0];
   if (path == 2) {
     const int n0 = mesh->n[0], n1 = mesh->n[1];

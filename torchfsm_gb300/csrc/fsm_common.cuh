@@ -333,10 +333,10 @@ struct FsmPlan {
   // per column tile of the register axis-0 pass (W adjacent inner columns): 1 where every column
   // is dealiased, so that the next-stage fields built there are zero (null: no such pass)
   uint8_t* tile_zero = nullptr;
-  // 2D plane passes: the leading last-axis columns of the stage fields that the row pass reads.
-  // Below h when the dealias mask keeps the prefix of n1/3 + 1 columns (the 2/3 rule) and the
-  // register passes run both axes: the fields beyond it are zero, so the column pass does not
-  // store them and the row pass does not load them.
+  // 2D and 3D passes: the leading last-axis columns of the stage fields that the passes exchange.
+  // Below h when the dealias mask keeps the prefix of n/3 + 1 columns (the 2/3 rule): the fields
+  // beyond it are zero, so they are neither stored nor loaded (3D: nor the kept columns of middle-axis
+  // modes that the mask drops).
   int hk = 0;
   // Row pitch (complex entries) and field stride of the stage fields and products (workspace
   // arrays exchanged between the passes). 2D register passes: n1/2 + 1 rounded up to even, so that

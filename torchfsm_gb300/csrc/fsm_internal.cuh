@@ -43,7 +43,7 @@ struct StepArgs {
   int64_t S;
   int H;
   const uint8_t* tile_zero;  // register axis-0 pass: column tiles whose next-stage fields are zero
-  int hk;                     // 2D: last-axis columns of the stage fields stored and read (FsmPlan::hk)
+  int hk;                     // last-axis columns of the stage fields stored and read (FsmPlan::hk)
   int64_t wp, ms;             // row pitch and field stride of mid / prod (FsmPlan::wp, ms)
   const int32_t* tab_entry;   // per sample: its coefficient-table entry (serving), or null
 };

@@ -4,14 +4,18 @@
 
 namespace fsm {
 
+// channel groups of a program (grid.z)
+template <int KIND, int DIM>
+constexpr int kGroups = RegKind<KIND, DIM>::C / RegKind<KIND, DIM>::CG;
+
 template <int NX, int KIND, int DIM>
 __global__ void __launch_bounds__(256) k_axis0_r(StepArgs a) {
-  axis0_body<NX, KIND, DIM, false>(a, blockIdx.x, blockIdx.y);
+  axis0_body<NX, KIND, DIM, false>(a, blockIdx.x, blockIdx.y, kGroups<KIND, DIM> > 1 ? blockIdx.z : 0);
 }
 
 template <int NX, int KIND, int DIM>
 __global__ void __launch_bounds__(256, 2) k_axis0_r2(StepArgs a) {
-  axis0_body<NX, KIND, DIM, true>(a, blockIdx.x, blockIdx.y);
+  axis0_body<NX, KIND, DIM, true>(a, blockIdx.x, blockIdx.y, kGroups<KIND, DIM> > 1 ? blockIdx.z : 0);
 }
 
 template <int NX, int KIND, int DIM, bool FAST>
@@ -20,7 +24,7 @@ static int launch_axis0_r_mode(const StepArgs& a, cudaStream_t st) {
   using K = RegKind<KIND, DIM>;
   const size_t smem = (size_t)(NX + (K::CG + 1) * Cfg::W * Cfg::P) * sizeof(float2);
   const int64_t inner = a.S / NX;
-  dim3 grid((unsigned)((inner + Cfg::W - 1) / Cfg::W), a.B);
+  dim3 grid((unsigned)((inner + Cfg::W - 1) / Cfg::W), a.B, kGroups<KIND, DIM>);
   if constexpr (FAST) {
     int rc = prep_smem(k_axis0_r2<NX, KIND, DIM>, smem);
     if (rc) return rc;

@@ -28,10 +28,14 @@ __device__ __forceinline__ void axis0_multi_body(const PlaneMulti& m) {
   int local = 0;
   const int j = multi_entry(m, &local);
   const int tile = local % m.gx[j], b = local / m.gx[j];
-  switch (m.n[j]) {
-    case 64: axis0_body<64, KIND, 2, FAST>(m.a[j], tile, b); break;
-    case 128: axis0_body<128, KIND, 2, FAST>(m.a[j], tile, b); break;
-    case 256: axis0_body<256, KIND, 2, FAST>(m.a[j], tile, b); break;
+#pragma unroll 1
+  for (int cg = 0; cg < RegKind<KIND, 2>::C / RegKind<KIND, 2>::CG; ++cg) {
+    if (cg) __syncthreads();  // the group before is done with the tiles
+    switch (m.n[j]) {
+      case 64: axis0_body<64, KIND, 2, FAST>(m.a[j], tile, b, cg); break;
+      case 128: axis0_body<128, KIND, 2, FAST>(m.a[j], tile, b, cg); break;
+      case 256: axis0_body<256, KIND, 2, FAST>(m.a[j], tile, b, cg); break;
+    }
   }
 }
 

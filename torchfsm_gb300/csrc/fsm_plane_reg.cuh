@@ -303,8 +303,11 @@ __device__ __forceinline__ void axis0_update(const StepArgs& a, float2* __restri
 // FAST: a SETDRK4 stage launch of a vorticity or convection program (channel groups of one
 // channel; the hoisted update, two CTAs per SM, k_axis0_r2); otherwise any scheme, the priming
 // launch included (k_axis0_r).
+// One channel group cg: a CTA of its own per group (grid.z), so that the channels of a velocity run
+// side by side instead of one after the other (3D Burgers 64^3 x 3: the x pass had 198 CTAs of three
+// channels each; with the kept columns of the 3D passes 7.03 -> 5.60 ms per 20 steps).
 template <int NX, int KIND, int DIM, bool FAST>
-__device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b) {
+__device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, int cg) {
   using Cfg = ColCfg<NX>;
   using K = RegKind<KIND, DIM>;
   constexpr int T = Cfg::T, E = Cfg::E, W = Cfg::W, P = Cfg::P, C = K::C, CG = K::CG;
@@ -324,120 +327,124 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b) {
   const int64_t gcol = c0 + g;
   const PointK<DIM> gk = point_k<DIM>(a, 0, gcol < inner ? gcol : inner - 1);
 
-  for (int cg = 0; cg < C / CG; ++cg) {
-    if (a.stage >= 0) {
-      for (int f = 0; f < CG; ++f) {
-        const float2* src = a.prod + ((int64_t)b * a.n_prod + cg * CG + f) * a.ms;
-        // all loads of the tile are issued before the shared-memory stores
-        float2 buf[NX * W / 256];
+  if (a.stage >= 0) {
+    for (int f = 0; f < CG; ++f) {
+      const float2* src = a.prod + ((int64_t)b * a.n_prod + cg * CG + f) * a.ms;
+      // all loads of the tile are issued before the shared-memory stores
+      float2 buf[NX * W / 256];
 #pragma unroll
-        for (int it = 0; it < NX * W / 256; ++it) {
-          const int idx = threadIdx.x + it * 256;
-          const int row = idx / W, col = idx % W;
-          if (c0 + col < inner) buf[it] = src[(int64_t)row * a.wp + c0 + col];
-        }
-#pragma unroll
-        for (int it = 0; it < NX * W / 256; ++it) {
-          const int idx = threadIdx.x + it * 256;
-          const int row = idx / W, col = idx % W;
-          if (c0 + col < inner) tileA[(f * W + col) * P + row] = buf[it];
-        }
+      for (int it = 0; it < NX * W / 256; ++it) {
+        const int idx = threadIdx.x + it * 256;
+        const int row = idx / W, col = idx % W;
+        if (c0 + col < inner) buf[it] = src[(int64_t)row * a.wp + c0 + col];
       }
-      __syncthreads();
-      for (int f = 0; f < CG; ++f) {
-        float2* colp = tileA + (f * W + g) * P;
-        float2 v[E];
 #pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = colp[t + T * j];
-        reg_fft<NX, false>(v, tileB + g * P, twt, t);
-#pragma unroll
-        for (int j = 0; j < E; ++j) colp[t + T * j] = v[j];
+      for (int it = 0; it < NX * W / 256; ++it) {
+        const int idx = threadIdx.x + it * 256;
+        const int row = idx / W, col = idx % W;
+        if (c0 + col < inner) tileA[(f * W + col) * P + row] = buf[it];
       }
     }
     __syncthreads();
-
-    if constexpr (FAST) {
-      switch (a.stage) {
-        case 0: axis0_update_hoisted<NX, KIND, DIM, 0>(a, tileA, b, c0, cg, last); break;
-        case 1: axis0_update_hoisted<NX, KIND, DIM, 1>(a, tileA, b, c0, cg, last); break;
-        case 2: axis0_update_hoisted<NX, KIND, DIM, 2>(a, tileA, b, c0, cg, last); break;
-        default: axis0_update_hoisted<NX, KIND, DIM, 3>(a, tileA, b, c0, cg, last); break;
-      }
-    } else if (a.stage >= 0 && a.integ == FSM_SETDRK4) {
-      switch (a.stage) {
-        case 0: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 0>(a, tileA, b, c0, cg, last); break;
-        case 1: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 1>(a, tileA, b, c0, cg, last); break;
-        case 2: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 2>(a, tileA, b, c0, cg, last); break;
-        default: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 3>(a, tileA, b, c0, cg, last); break;
-      }
-    } else {
-      axis0_update<NX, KIND, DIM, -1, -1>(a, tileA, b, c0, cg, last);
-    }
-    if (!a.emit) continue;  // uniform: no further barriers in this group
-    // 2D: columns from hk on are dealiased and the row pass does not read them: nothing to store
-    if (c0 >= ((DIM == 2) ? (int64_t)a.hk : inner)) continue;  // uniform
-    if (a.tile_zero && a.tile_zero[tile]) {
-      // every column of this tile is dealiased: the next-stage fields are zero here, written
-      // directly (coalesced rows of W columns) without the transforms
-      constexpr int NMO = (KIND == FSM_NL_CONVECTION) ? 2 : K::NMG;  // fields of this channel group
-      const int m0 = (KIND == FSM_NL_CONVECTION) ? cg * 2 : 0;
-#pragma unroll 1
-      for (int mf = 0; mf < NMO; ++mf) {
-        float2* dst = a.mid + ((int64_t)b * a.n_mid + m0 + mf) * a.ms;
-#pragma unroll
-        for (int it = 0; it < NX * W / 256; ++it) {
-          const int idx = threadIdx.x + it * 256;
-          const int row = idx / W, cc = idx % W;
-          if (c0 + cc < inner) dst[(int64_t)row * a.wp + c0 + cc] = make_float2(0.f, 0.f);
-        }
-      }
-      continue;  // uniform across the CTA
-    }
-    __syncthreads();
-
-    // Next-stage fields: each group transforms its own column into tileB, then the CTA
-    // stores the tile with a coalesced mapping (rows of W adjacent columns).
-    for (int mf = 0; mf < K::NMG; ++mf) {
-      const int f = (KIND == FSM_NL_VORTICITY || KIND == FSM_NL_KS) ? 0 : (mf >> 1);
-      const float2* colp = tileA + (f * W + g) * P;
+    for (int f = 0; f < CG; ++f) {
+      float2* colp = tileA + (f * W + g) * P;
       float2 v[E];
 #pragma unroll
-      for (int j = 0; j < E; ++j) {
-        const float2 d = colp[t + T * j];
-        const float kxv = kxr[j];
-        float2 x;
-        if (KIND == FSM_NL_VORTICITY) {
-          // 0: psi = -w/lap, 1: i kx psi, 2: w, 3: i kx w
-          if (mf < 2) {
-            const float lap = -(kxv * kxv + gk.ky * gk.ky);
-            // fast division: within 2 ulp for |lap| below 2^126, far above any mesh's 2 (pi NX / L)^2
-            const float il = (lap == 0.f) ? 1.f : __fdividef(1.f, lap);
-            const float2 psi = cscale(d, -il);
-            x = (mf == 0) ? psi : cscale(cmuli(psi), kxv);
-          } else {
-            x = (mf == 2) ? d : cscale(cmuli(d), kxv);
-          }
-        } else {
-          // KS: 0: phi, 1: i kx phi; convection (per channel): u_c, i kx u_c
-          x = (mf & 1) ? cscale(cmuli(d), kxv) : d;
-        }
-        v[j] = x;
-      }
-      float2* ob = tileB + g * P;
-      reg_fft<NX, true>(v, ob, twt, t);
+      for (int j = 0; j < E; ++j) v[j] = colp[t + T * j];
+      reg_fft<NX, false>(v, tileB + g * P, twt, t);
 #pragma unroll
-      for (int j = 0; j < E; ++j) ob[t + T * j] = v[j];
-      __syncthreads();
-      const int mout = (KIND == FSM_NL_CONVECTION) ? cg * 2 + mf : mf;
-      float2* dst = a.mid + ((int64_t)b * a.n_mid + mout) * a.ms;
+      for (int j = 0; j < E; ++j) colp[t + T * j] = v[j];
+    }
+  }
+  __syncthreads();
+
+  if constexpr (FAST) {
+    switch (a.stage) {
+      case 0: axis0_update_hoisted<NX, KIND, DIM, 0>(a, tileA, b, c0, cg, last); break;
+      case 1: axis0_update_hoisted<NX, KIND, DIM, 1>(a, tileA, b, c0, cg, last); break;
+      case 2: axis0_update_hoisted<NX, KIND, DIM, 2>(a, tileA, b, c0, cg, last); break;
+      default: axis0_update_hoisted<NX, KIND, DIM, 3>(a, tileA, b, c0, cg, last); break;
+    }
+  } else if (a.stage >= 0 && a.integ == FSM_SETDRK4) {
+    switch (a.stage) {
+      case 0: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 0>(a, tileA, b, c0, cg, last); break;
+      case 1: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 1>(a, tileA, b, c0, cg, last); break;
+      case 2: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 2>(a, tileA, b, c0, cg, last); break;
+      default: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 3>(a, tileA, b, c0, cg, last); break;
+    }
+  } else {
+    axis0_update<NX, KIND, DIM, -1, -1>(a, tileA, b, c0, cg, last);
+  }
+  if (!a.emit) return;  // uniform
+  // 2D: columns from hk on are dealiased and the row pass does not read them: nothing to store.
+  // 3D: the next passes read the columns (jm, jl) with jm kept and jl < hk.
+  if (DIM == 2 && c0 >= (int64_t)a.hk) return;  // uniform
+  if (a.tile_zero && a.tile_zero[tile]) {
+    if (DIM == 3 && a.hk < a.H) return;
+    // every column of this tile is dealiased: the next-stage fields are zero here, written
+    // directly (coalesced rows of W columns) without the transforms
+    constexpr int NMO = (KIND == FSM_NL_CONVECTION) ? 2 : K::NMG;  // fields of this channel group
+    const int m0 = (KIND == FSM_NL_CONVECTION) ? cg * 2 : 0;
+#pragma unroll 1
+    for (int mf = 0; mf < NMO; ++mf) {
+      float2* dst = a.mid + ((int64_t)b * a.n_mid + m0 + mf) * a.ms;
 #pragma unroll
       for (int it = 0; it < NX * W / 256; ++it) {
         const int idx = threadIdx.x + it * 256;
         const int row = idx / W, cc = idx % W;
-        if (c0 + cc < ((DIM == 2) ? (int64_t)a.hk : inner)) dst[(int64_t)row * a.wp + c0 + cc] = tileB[cc * P + row];
+        if (c0 + cc < inner) dst[(int64_t)row * a.wp + c0 + cc] = make_float2(0.f, 0.f);
       }
-      __syncthreads();
     }
+    return;  // uniform across the CTA
+  }
+  __syncthreads();
+  const int64_t sj = c0 + threadIdx.x % W;  // the column this thread stores
+  bool live = sj < inner;
+  if (DIM == 2) live = sj < (int64_t)a.hk;
+  else if (live) live = (int)(sj % a.H) < a.hk && (a.hk == a.H || a.keepm[(int)(sj / a.H)]);
+
+  // Next-stage fields: each group transforms its own column into tileB, then the CTA
+  // stores the tile with a coalesced mapping (rows of W adjacent columns).
+  for (int mf = 0; mf < K::NMG; ++mf) {
+    const int f = (KIND == FSM_NL_VORTICITY || KIND == FSM_NL_KS) ? 0 : (mf >> 1);
+    const float2* colp = tileA + (f * W + g) * P;
+    float2 v[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+      const float2 d = colp[t + T * j];
+      const float kxv = kxr[j];
+      float2 x;
+      if (KIND == FSM_NL_VORTICITY) {
+        // 0: psi = -w/lap, 1: i kx psi, 2: w, 3: i kx w
+        if (mf < 2) {
+          const float lap = -(kxv * kxv + gk.ky * gk.ky);
+          // fast division: within 2 ulp for |lap| below 2^126, far above any mesh's 2 (pi NX / L)^2
+          const float il = (lap == 0.f) ? 1.f : __fdividef(1.f, lap);
+          const float2 psi = cscale(d, -il);
+          x = (mf == 0) ? psi : cscale(cmuli(psi), kxv);
+        } else {
+          x = (mf == 2) ? d : cscale(cmuli(d), kxv);
+        }
+      } else {
+        // KS: 0: phi, 1: i kx phi; convection (per channel): u_c, i kx u_c
+        x = (mf & 1) ? cscale(cmuli(d), kxv) : d;
+      }
+      v[j] = x;
+    }
+    float2* ob = tileB + g * P;
+    reg_fft<NX, true>(v, ob, twt, t);
+#pragma unroll
+    for (int j = 0; j < E; ++j) ob[t + T * j] = v[j];
+    __syncthreads();
+    const int mout = (KIND == FSM_NL_CONVECTION) ? cg * 2 + mf : mf;
+    float2* dst = a.mid + ((int64_t)b * a.n_mid + mout) * a.ms;
+#pragma unroll
+    for (int it = 0; it < NX * W / 256; ++it) {
+      const int idx = threadIdx.x + it * 256;
+      const int row = idx / W, cc = idx % W;
+      if (live) dst[(int64_t)row * a.wp + c0 + cc] = tileB[cc * P + row];
+    }
+    __syncthreads();
   }
 }
 
@@ -483,19 +490,6 @@ __device__ __forceinline__ void split_store_r(const float2 (&zp)[RegShape<NY>::E
       out1[k] = cscale(cmulmi(csub(zp[j], zm)), 0.5f);
     }
   }
-}
-
-// Whether every lane of register j (indices k = t + T j, folded to kk = min(k, NY - k)) lies at
-// or beyond the kept prefix HK of the last axis: such registers hold zeros and load nothing.
-template <int NY, int T, int HK>
-__device__ __forceinline__ constexpr bool reg_dead(int j) {
-  int mn = NY;
-  for (int t = 0; t < T; ++t) {
-    const int k = t + T * j;
-    const int kk = k <= NY / 2 ? k : NY - k;
-    mn = kk < mn ? kk : mn;
-  }
-  return mn >= HK;
 }
 
 // HK: the stage fields' stored columns (FsmPlan::hk), NY/2 + 1 when every column is stored.

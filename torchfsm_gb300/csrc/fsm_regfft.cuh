@@ -189,4 +189,17 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::E], float2* __r
   }
 }
 
+// Whether every lane of register j (indices k = t + T j, folded to kk = min(k, NY - k)) lies at
+// or beyond the kept prefix HK of the last axis: such registers hold zeros and load nothing.
+template <int NY, int T, int HK>
+__device__ __forceinline__ constexpr bool reg_dead(int j) {
+  int mn = NY;
+  for (int t = 0; t < T; ++t) {
+    const int k = t + T * j;
+    const int kk = k <= NY / 2 ? k : NY - k;
+    mn = kk < mn ? kk : mn;
+  }
+  return mn >= HK;
+}
+
 }  // namespace fsm

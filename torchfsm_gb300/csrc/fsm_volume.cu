@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) k_axis1_inv_r(StepArgs a) {
   float2* tB = tA + W * P;  // X (i kx u_c)     -> Y(X (i kx u_c))
   float2* tC = tB + W * P;  //                  -> Y(X u_c)
   const int g = threadIdx.x / T, t = threadIdx.x % T;
-  const int H = a.H;
+  const int H = a.H, HK = a.hk;  // columns beyond HK are dealiased: zero, neither read nor written
   const int x = blockIdx.y;
   const int groups_c = a.n_mid / 2;
   const int b = blockIdx.z / groups_c, c = blockIdx.z % groups_c;
@@ -127,7 +127,9 @@ __global__ void __launch_bounds__(256) k_axis1_inv_r(StepArgs a) {
     for (int it = 0; it < NY * W / 256; ++it) {
       const int idx = threadIdx.x + it * 256;
       const int row = idx / W, col = idx % W;
-      if (c0 + col < H) {
+      b0[it] = b1[it] = make_float2(0.f, 0.f);
+      // rows that the mask drops are not stored by the x pass (FsmPlan::hk)
+      if (c0 + col < HK && (HK == H || a.keepm[row])) {
         b0[it] = in0[(int64_t)row * H + c0 + col];
         b1[it] = in1[(int64_t)row * H + c0 + col];
       }
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(256) k_axis1_inv_r(StepArgs a) {
     for (int it = 0; it < NY * W / 256; ++it) {
       const int idx = threadIdx.x + it * 256;
       const int row = idx / W, col = idx % W;
-      if (c0 + col < H) {
+      if (c0 + col < HK) {
         tA[col * P + row] = b0[it];
         tB[col * P + row] = b1[it];
       }
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(256) k_axis1_inv_r(StepArgs a) {
   float2* out = a.mid2 + ((int64_t)b * a.n_mid2 + 3 * c) * S + (int64_t)x * plane;
   for (int idx = threadIdx.x; idx < NY * W; idx += 256) {
     const int row = idx / W, col = idx % W;
-    if (c0 + col < H) {
+    if (c0 + col < HK) {
       const int64_t o = (int64_t)row * H + c0 + col;
       out[o] = tC[col * P + row];          // Y(X u_c)
       out[S + o] = tB[col * P + row];      // Y(X (i kx u_c))
@@ -192,20 +194,25 @@ __device__ __forceinline__ float2 herm_z3(float2 A, float2 B, bool selfc, bool h
 
 // Build Z = A + i B (Hermitian extension over the row) from two mid2 fields;
 // `da`/`db` apply the i kz factor to A / B.
-template <int NZ>
+template <int NZ, int HK>
 __device__ __forceinline__ void build_row(float2 (&Z)[RegShape<NZ>::E], const float2* __restrict__ fa,
                                           const float2* __restrict__ fb, bool da, bool db, const float* __restrict__ kz,
                                           int t) {
   constexpr int T = RegShape<NZ>::T, E = RegShape<NZ>::E;
 #pragma unroll
   for (int j = 0; j < E; ++j) {
+    if (reg_dead<NZ, T, HK>(j)) {  // every lane beyond the kept prefix
+      Z[j] = make_float2(0.f, 0.f);
+      continue;
+    }
     const int k = t + T * j;
     const bool hi = k > NZ / 2;
     const int kk = hi ? NZ - k : k;
     const bool selfc = (kk == 0) || (kk == NZ / 2);
+    const bool live = HK > NZ / 2 || kk < HK;
     const float kzv = kz[kk];
-    float2 A = fa ? fa[kk] : make_float2(0.f, 0.f);
-    float2 B = fb ? fb[kk] : make_float2(0.f, 0.f);
+    float2 A = fa && live ? fa[kk] : make_float2(0.f, 0.f);
+    float2 B = fb && live ? fb[kk] : make_float2(0.f, 0.f);
     if (da) A = cscale(cmuli(A), kzv);
     if (db) B = cscale(cmuli(B), kzv);
     Z[j] = herm_z3(A, B, selfc, hi);
@@ -234,7 +241,7 @@ __device__ __forceinline__ void split_one(const float2 (&zp)[RegShape<NZ>::E], i
   }
 }
 
-template <int NZ, int KIND>
+template <int NZ, int KIND, int HK>
 __global__ void __launch_bounds__(256, 2) k_axis2_r(StepArgs a) {
   using RS = RegShape<NZ>;
   constexpr int T = RS::T, E = RS::E, SCR = reg_scratch<NZ>();
@@ -266,36 +273,36 @@ __global__ void __launch_bounds__(256, 2) k_axis2_r(StepArgs a) {
 #pragma unroll
       for (int i = 0; i < 9; ++i) F[i] = m2 + i * S + roff;
       float c0v[E], c1v[E], c2v[E];
-      build_row<NZ>(Z, F[0], F[3], false, false, kz, t);  // u0 + i u1
+      build_row<NZ, HK>(Z, F[0], F[3], false, false, kz, t);  // u0 + i u1
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         ust[t + T * j] = Z[j].x;
         ust[NZ + t + T * j] = Z[j].y;
       }
-      build_row<NZ>(Z, F[6], F[1], false, false, kz, t);  // u2 + i dx u0
+      build_row<NZ, HK>(Z, F[6], F[1], false, false, kz, t);  // u2 + i dx u0
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         ust[2 * NZ + t + T * j] = Z[j].x;
         c0v[j] = ust[t + T * j] * Z[j].y;
       }
-      build_row<NZ>(Z, F[2], F[0], false, true, kz, t);  // dy u0 + i dz u0
+      build_row<NZ, HK>(Z, F[2], F[0], false, true, kz, t);  // dy u0 + i dz u0
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) c0v[j] += ust[NZ + t + T * j] * Z[j].x + ust[2 * NZ + t + T * j] * Z[j].y;
-      build_row<NZ>(Z, F[4], F[5], false, false, kz, t);  // dx u1 + i dy u1
+      build_row<NZ, HK>(Z, F[4], F[5], false, false, kz, t);  // dx u1 + i dy u1
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) c1v[j] = ust[t + T * j] * Z[j].x + ust[NZ + t + T * j] * Z[j].y;
-      build_row<NZ>(Z, F[3], F[7], true, false, kz, t);  // dz u1 + i dx u2
+      build_row<NZ, HK>(Z, F[3], F[7], true, false, kz, t);  // dz u1 + i dx u2
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         c1v[j] += ust[2 * NZ + t + T * j] * Z[j].x;
         c2v[j] = ust[t + T * j] * Z[j].y;
       }
-      build_row<NZ>(Z, F[8], F[6], false, true, kz, t);  // dy u2 + i dz u2
+      build_row<NZ, HK>(Z, F[8], F[6], false, true, kz, t);  // dy u2 + i dz u2
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) c2v[j] += ust[NZ + t + T * j] * Z[j].x + ust[2 * NZ + t + T * j] * Z[j].y;
@@ -310,11 +317,11 @@ __global__ void __launch_bounds__(256, 2) k_axis2_r(StepArgs a) {
     } else {
       // KS: mid2 0: Y(X phi) -> dz via i kz, 1: -> dx phi, 2: -> dy phi
       float p[E];
-      build_row<NZ>(Z, m2 + S + roff, m2 + 2 * S + roff, false, false, kz, t);  // dx + i dy
+      build_row<NZ, HK>(Z, m2 + S + roff, m2 + 2 * S + roff, false, false, kz, t);  // dx + i dy
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) p[j] = 0.5f * (Z[j].x * Z[j].x + Z[j].y * Z[j].y);
-      build_row<NZ>(Z, m2 + roff, nullptr, true, false, kz, t);  // dz
+      build_row<NZ, HK>(Z, m2 + roff, nullptr, true, false, kz, t);  // dz
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) Z[j] = make_float2(p[j] + 0.5f * Z[j].x * Z[j].x, 0.f);
@@ -330,13 +337,13 @@ static int launch_axis1_inv(int n0, const StepArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)(NY + 3 * Cfg::W * Cfg::P) * sizeof(float2);
   int rc = prep_smem(k_axis1_inv_r<NY>, smem);
   if (rc) return rc;
-  dim3 grid((unsigned)((a.H + Cfg::W - 1) / Cfg::W), (unsigned)n0, (unsigned)(a.B * (a.n_mid / 2)));
+  dim3 grid((unsigned)((a.hk + Cfg::W - 1) / Cfg::W), (unsigned)n0, (unsigned)(a.B * (a.n_mid / 2)));
   k_axis1_inv_r<NY><<<grid, 256, smem, st>>>(a);
   return cuda_check(cudaGetLastError(), "k_axis1_inv_r");
 }
 
-template <int NZ, int KIND>
-static int launch_axis2(const StepArgs& a, cudaStream_t st) {
+template <int NZ, int KIND, int HK>
+static int launch_axis2_hk(const StepArgs& a, cudaStream_t st) {
   using RS = RegShape<NZ>;
   constexpr int H = NZ / 2 + 1;
   const int64_t rows = a.S / H;
@@ -344,11 +351,18 @@ static int launch_axis2(const StepArgs& a, cudaStream_t st) {
   int threads = (int)((groups_needed * RS::T < 256) ? groups_needed * RS::T : 256);
   const int groups = threads / RS::T;
   const size_t smem = (size_t)(NZ + groups * reg_scratch<NZ>()) * sizeof(float2) + (size_t)groups * 3 * NZ * sizeof(float);
-  int rc = prep_smem(k_axis2_r<NZ, KIND>, smem);
+  int rc = prep_smem(k_axis2_r<NZ, KIND, HK>, smem);
   if (rc) return rc;
   dim3 grid((unsigned)((groups_needed + groups - 1) / groups), a.B);
-  k_axis2_r<NZ, KIND><<<grid, threads, smem, st>>>(a);
+  k_axis2_r<NZ, KIND, HK><<<grid, threads, smem, st>>>(a);
   return cuda_check(cudaGetLastError(), "k_axis2_r");
+}
+
+// The 2/3 rule's prefix (NZ/3 + 1 columns) or every column.
+template <int NZ, int KIND>
+static int launch_axis2(const StepArgs& a, cudaStream_t st) {
+  if (a.hk == NZ / 3 + 1) return launch_axis2_hk<NZ, KIND, NZ / 3 + 1>(a, st);
+  return launch_axis2_hk<NZ, KIND, NZ / 2 + 1>(a, st);
 }
 
 int launch_volume_axis1_inv(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
