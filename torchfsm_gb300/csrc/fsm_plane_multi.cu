@@ -78,7 +78,7 @@ namespace {
 template <int N, int KIND>
 void col_shape(const StepArgs& a, size_t* smem, int* per_sample) {
   using Cfg = ColCfg<N>;
-  *smem = (size_t)(N + (RegKind<KIND, 2>::CG + 1) * Cfg::W * Cfg::P) * sizeof(float2);
+  *smem = (size_t)Cfg::WORDS * sizeof(float2);
   *per_sample = (int)((a.S / N + Cfg::W - 1) / Cfg::W);
 }
 

@@ -29,11 +29,9 @@
 // transform of the two rows' products packed as one complex row and splits
 // the half spectra with one shuffle per output register.
 //
-// Column pass: a CTA owns W = 256/T adjacent ky columns of one sample. The
-// products are staged into a padded column-major tile (coalesced loads), each
-// group transforms one column, the stage update runs with a coalesced point
-// mapping, and each next-stage field is transformed per column and staged
-// through a second tile for coalesced stores.
+// Column pass: a CTA owns W = 256/T adjacent ky columns of one sample; a thread holds T-strided rows
+// of one column in registers from the products through the update to the next-stage fields, with a
+// warp's lanes on adjacent columns, so every global access is coalesced without staging.
 #pragma once
 
 #include "fsm_internal.cuh"
@@ -56,10 +54,78 @@ struct ColCfg {
   using RS = RegShape<NX>;
   static constexpr int T = RS::T;
   static constexpr int E = RS::E;
-  static constexpr int W = 256 / T;
-  static constexpr int NEED = (NX > reg_scratch<NX>()) ? NX : reg_scratch<NX>();
-  static constexpr int P = NEED | 1;  // odd pitch: a row across W columns hits W distinct banks
+  static constexpr int W = 256 / T;  // columns of a CTA
+  // words of an exchange buffer (512 points: one row of padding per 16)
+  static constexpr int XB = (NX == 512 ? 512 + 32 : E * T) * W;
+  // shared memory (float2): twiddles, kx, two exchange buffers
+  static constexpr int WORDS = NX + NX / 2 + 2 * XB;
 };
+
+// x transform of a CTA's W columns: thread (t, g) = threadIdx / W, threadIdx % W holds rows t + T j of
+// column g in registers on entry and exit (fsm_regfft.cuh's passes). The lanes of a warp are adjacent
+// columns, so that global loads and stores of those registers are coalesced as they are, and so are
+// the exchange's accesses to shared memory; the price is a CTA barrier per exchange, one each with
+// two buffers in turn (par selects the next).
+template <int NX, bool INV>
+__device__ __forceinline__ void col_fft(float2 (&v)[RegShape<NX>::E], float2* __restrict__ buf, int& par,
+                                        const float2* __restrict__ twt, int t, int g) {
+  using Cfg = ColCfg<NX>;
+  constexpr int T = Cfg::T, E = Cfg::E, W = Cfg::W;
+  auto tw = [&](float2 a, float2 w) {
+    if (INV) w.y = -w.y;
+    return cmul(a, w);
+  };
+  float2* x = buf + par * Cfg::XB + g;
+  par ^= 1;
+  if constexpr (NX == 512) {
+    auto pad = [](int i) { return (i + (i >> 4)) * W; };
+    float2* y = buf + par * Cfg::XB + g;
+    par ^= 1;
+    dft16<INV>(v);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[(17 * t + j) * W] = v[j];
+    __syncthreads();
+    const int k2 = t & 15;
+    const float2 w2 = twt[k2];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      v[2 * b] = x[pad(t + 32 * b)];
+      v[2 * b + 1] = tw(x[pad(t + 32 * b + 256)], w2);
+      dft2<INV>(v + 2 * b);
+    }
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const int base = (t + 32 * b - k2) * 2 + k2;
+      y[pad(base)] = v[2 * b];
+      y[pad(base + 16)] = v[2 * b + 1];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      v[j] = y[pad(t + 32 * j)];
+      if (j > 0) v[j] = tw(v[j], twt[16 + 32 * (j - 1) + t]);
+    }
+    dft16<INV>(v);
+  } else {
+    constexpr int PER = E / T;
+    dft_reg<E, INV>(v);
+#pragma unroll
+    for (int m = 1; m < E; ++m) v[m] = tw(v[m], twt[m * T + t]);
+#pragma unroll
+    for (int m = 0; m < E; ++m) x[(m * T + t) * W] = v[m];
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int m = t + p * T;
+      float2 w[T];
+#pragma unroll
+      for (int tt = 0; tt < T; ++tt) w[tt] = x[(m * T + tt) * W];
+      dft_reg<T, INV>(w);
+#pragma unroll
+      for (int k = 0; k < T; ++k) v[p + PER * k] = w[k];
+    }
+  }
+}
 
 // Wavenumbers and dealias factor of the point (row, inner index j). 2D: j is
 // the last-axis index; 3D: j = jm * H + jl (middle, last axis).
@@ -166,285 +232,312 @@ __device__ __forceinline__ float2 setdrk4_pre(float2 nv, float2 ua, float2 ub, c
   }
 }
 
-// Phase 2 of k_axis0_r for SETDRK4 stages of one-channel groups: the state operands the thread's
-// points need from HBM (u at stages 0 and 1, acc at 1, 2 and 3, q at 2) are loaded first for a
-// group of points, in one round, then those points are updated with their table loads (which hit
-// L2). Loading them four points at a time left four rounds of HBM latency in each CTA's critical
-// path (on 2D vorticity 256^2 x 64 the column pass went from 55 to 43 us per launch).
+// The SETDRK4 stage update of a thread's points (rows t + T j of its column) of a one-channel group,
+// N_s in v, the next stage's input out. o1 holds the operand loaded ahead of the forward transform
+// (u at stages 0 and 1, acc at stages 2 and 3), so that its latency passes behind the transform.
 template <int NX, int KIND, int DIM, int STG>
-__device__ __forceinline__ void axis0_update_hoisted(const StepArgs& a, float2* __restrict__ tileA, int b, int64_t c0,
+__device__ __forceinline__ void axis0_update_hoisted(const StepArgs& a, float2 (&v)[RegShape<NX>::E],
+                                                     const float2 (&o1)[RegShape<NX>::E], int b, int64_t j0, int t,
                                                      int cg, bool last) {
-  using Cfg = ColCfg<NX>;
   using K = RegKind<KIND, DIM>;
-  constexpr int W = Cfg::W, P = Cfg::P, C = K::C;
-  constexpr int PPT = NX * W / 256, RSTEP = 256 / W;
-  const int64_t S = a.S;
-  const int64_t inner = S / NX;
-  const int col = threadIdx.x % W, row0 = threadIdx.x / W;
-  const int64_t j = c0 + col;
-  if (j >= inner) return;
-  const int c = cg;
-  float2* __restrict__ up = a.state + ((int64_t)b * C + c) * S + j;
-  float2* __restrict__ accp = a.aux + ((int64_t)b * a.n_aux * C + c) * S + j;
-  float2* __restrict__ qp = a.aux + ((int64_t)b * a.n_aux * C + C + c) * S + j;
-  const float2* __restrict__ tab = a.tab + (tab_batch(a, b) * a.lin_ch + (a.lin_ch > 1 ? c : 0)) * S + j;
-  const float2* __restrict__ srcp =
-      a.src ? a.src + ((int64_t)(a.src_batch > 1 ? b : 0) * C + c) * S + j : nullptr;
-  const float2* __restrict__ o1p = (STG <= 1) ? up : accp;
+  constexpr int T = RegShape<NX>::T, E = RegShape<NX>::E, C = K::C;
+  const int64_t S = a.S, inner = S / NX;
+  const int64_t off = ((int64_t)b * C + cg) * S + j0;
+  float2* __restrict__ up = a.state + off;
+  float2* __restrict__ accp = a.aux + ((int64_t)b * a.n_aux * C + cg) * S + j0;
+  float2* __restrict__ qp = accp + (int64_t)C * S;
+  const float2* __restrict__ tab = a.tab + (tab_batch(a, b) * a.lin_ch + (a.lin_ch > 1 ? cg : 0)) * S + j0;
+  const float2* __restrict__ srcp = a.src ? a.src + ((int64_t)(a.src_batch > 1 ? b : 0) * C + cg) * S + j0 : nullptr;
   const float2* __restrict__ o2p = (STG == 1) ? accp : qp;
-  // operands of HALF points at a time, one HBM round per group: eight points (vorticity) and four
-  // (convection, whose kernel holds more) keep the kernels inside two CTAs' registers per SM
-  constexpr int HMAX = (KIND == FSM_NL_CONVECTION) ? 4 : 8;
-  constexpr int HALF = PPT > HMAX ? HMAX : PPT;
-#pragma unroll 1
-  for (int h0 = 0; h0 < PPT; h0 += HALF) {
-  float2 o1[HALF], o2[HALF];
+  // The operands of HALF points are loaded in one batch (one round of memory latency each half). The
+  // SETDRK coefficients are real (k_phi_tables): only the exponentials are read as complex.
+  constexpr int HALF = E > 8 ? 8 : E;
 #pragma unroll
-  for (int ih = 0; ih < HALF; ++ih) {
-    const int64_t r = (int64_t)(row0 + RSTEP * (h0 + ih)) * inner;
-    o1[ih] = o1p[r];
-    if (STG == 1 || STG == 2) o2[ih] = o2p[r];
-  }
+  for (int h0 = 0; h0 < E; h0 += HALF) {
+    float2 o2[HALF], em[HALF], e2[HALF];
+    float ca[HALF], cb[HALF];
 #pragma unroll
-  for (int ih = 0; ih < HALF; ++ih) {
-    const int it = h0 + ih;
-    // the table loads of four points at a time: without this fence the compiler issues those of
-    // every point at once, beside the operands, and runs out of registers
-    
-    const int row = row0 + RSTEP * it;
-    const int64_t r = (int64_t)row * inner;
-    const PointK<DIM> pk = point_k<DIM>(a, row, j);
-    float2 nv = tileA[col * P + row];
-    if (KIND == FSM_NL_KS && (a.flags & FSM_FLAG_REMOVE_MEAN) && row == 0 && j == 0) nv = csub(nv, a.dc[0]);
-    nv = cscale(nv, a.coef);
-    if (srcp) nv = cadd(nv, srcp[r]);
-    float2 acc, q;
-    const float2 st = setdrk4_pre<STG>(nv, o1[ih], (STG == 1 || STG == 2) ? o2[ih] : o1[ih], tab + r, a.ts, acc, q);
-    if (STG <= 2) accp[r] = acc;
-    if (STG == 0) qp[r] = q;
-    if (STG == 3) {
-      up[r] = st;
-      if (a.slot >= 0 && last) a.traj[(((int64_t)b * a.n_frames + a.slot) * C + c) * S + r + j] = st;
+    for (int i = 0; i < HALF; ++i) {
+      const int64_t r = (int64_t)(t + T * (h0 + i)) * inner;
+      if (STG == 1 || STG == 2) o2[i] = o2p[r];
+      if (STG == 0) em[i] = tab[r];
+      if (STG <= 1) e2[i] = tab[r + a.ts];
+      if (STG <= 2) ca[i] = tab[r + 2 * a.ts].x;
+      if (STG == 0) cb[i] = tab[r + 3 * a.ts].x;
+      if (STG == 1 || STG == 2) cb[i] = tab[r + 4 * a.ts].x;
+      if (STG == 3) cb[i] = tab[r + 5 * a.ts].x;
     }
-    tileA[col * P + row] = cscale(st, pk.mask);
-  }
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      const int j = h0 + i, row = t + T * j;
+      const int64_t r = (int64_t)row * inner;
+      float2 nv = v[j];
+      if (KIND == FSM_NL_KS && (a.flags & FSM_FLAG_REMOVE_MEAN) && row == 0 && j0 == 0) nv = csub(nv, a.dc[0]);
+      nv = cscale(nv, a.coef);
+      if (srcp) nv = cadd(nv, srcp[r]);
+      float2 tb[6];
+      tb[0] = em[i];
+      tb[1] = e2[i];
+      tb[2] = make_float2(ca[i], 0.f);
+      tb[3] = tb[4] = tb[5] = make_float2(cb[i], 0.f);
+      float2 acc, q;
+      const float2 st = setdrk4_pre<STG>(nv, o1[j], (STG == 1 || STG == 2) ? o2[i] : o1[j], tb, 1, acc, q);
+      if (STG <= 2) accp[r] = acc;
+      if (STG == 0) qp[r] = q;
+      if (STG == 3) {
+        up[r] = st;
+        if (a.slot >= 0 && last) a.traj[(((int64_t)b * a.n_frames + a.slot) * C + cg) * S + r + j0] = st;
+      }
+      v[j] = st;
+    }
   }
 }
 
-// Phase 2 of k_axis0_r: the stage update at every point of the tile, in a coalesced point
-// mapping, leaving the masked next-stage field in tileA. INTEG/STG name the scheme and stage
-// at compile time (so that the loads of several points are issued together); -1 dispatches
-// at run time.
-template <int NX, int KIND, int DIM, int INTEG, int STG>
-__device__ __forceinline__ void axis0_update(const StepArgs& a, float2* __restrict__ tileA, int b, int64_t c0, int cg,
-                                             bool last) {
-  using Cfg = ColCfg<NX>;
+// N_s of a point's channels: the Leray projection, the KS batch mean, coefficient and source.
+template <int NX, int KIND, int DIM>
+__device__ __forceinline__ void axis0_nonlinear(const StepArgs& a, float2 (&nv)[RegKind<KIND, DIM>::CG], int b,
+                                                int64_t j0, int row, int cg) {
   using K = RegKind<KIND, DIM>;
-  constexpr int W = Cfg::W, P = Cfg::P, C = K::C, CG = K::CG;
-  const int64_t S = a.S;
-  const int64_t inner = S / NX;
-  const bool update = STG >= 0 || a.stage >= 0;  // false: the priming launch (mask and emit only)
-  // restrict-qualified views so that loads of later points may be issued ahead of the stores of earlier ones
+  constexpr int C = K::C, CG = K::CG;
+  if (KIND == FSM_NL_LERAY) nv_leray<DIM, CG>(nv, point_k<DIM>(a, row, j0), row, j0, a, NX);
+  if (KIND == FSM_NL_KS && (a.flags & FSM_FLAG_REMOVE_MEAN) && row == 0 && j0 == 0) nv[0] = csub(nv[0], a.dc[0]);
+#pragma unroll
+  for (int f = 0; f < CG; ++f) {
+    nv[f] = cscale(nv[f], a.coef);
+    if (a.src)
+      nv[f] = cadd(nv[f], a.src[((int64_t)(a.src_batch > 1 ? b : 0) * C + cg * CG + f) * a.S +
+                                (int64_t)row * (a.S / NX) + j0]);
+  }
+}
+
+// The stage update of a thread's points, all channels of the group, in registers: SETDRK4 stage STG
+// (INTEG FSM_SETDRK4), the right-hand side itself (FSM_APPLY), or the priming launch (STG -1), which
+// only reads the state.
+template <int NX, int KIND, int DIM, int INTEG, int STG>
+__device__ __forceinline__ void axis0_update(const StepArgs& a, float2 (&v)[RegKind<KIND, DIM>::CG][RegShape<NX>::E],
+                                             int b, int64_t j0, int t, int cg, bool last) {
+  using K = RegKind<KIND, DIM>;
+  constexpr int T = RegShape<NX>::T, E = RegShape<NX>::E, C = K::C, CG = K::CG;
+  const int64_t S = a.S, inner = S / NX;
   float2* __restrict__ state = a.state;
   float2* __restrict__ aux = a.aux;
   float2* __restrict__ traj = a.traj;
   const float2* __restrict__ tab = a.tab;
-  const float2* __restrict__ srcp = a.src;
-  constexpr int PPT = NX * W / 256;  // points per thread
-#pragma unroll 4
-  for (int it = 0; it < PPT; ++it) {
-    const int idx = threadIdx.x + it * 256;
-    const int row = idx / W, col = idx % W;
-    const int64_t j = c0 + col;
-    if (j >= inner) continue;
-    const int64_t sidx = (int64_t)row * inner + j;
-    const PointK<DIM> pk = point_k<DIM>(a, row, j);
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int row = t + T * i;
+    const int64_t sidx = (int64_t)row * inner + j0;
     float2 nv[CG];
-    if (update) {
+    if (STG >= 0) {
 #pragma unroll
-      for (int f = 0; f < CG; ++f) nv[f] = tileA[(f * W + col) * P + row];
-      if (KIND == FSM_NL_LERAY) nv_leray<DIM, CG>(nv, pk, row, j, a, NX);
-      if (KIND == FSM_NL_KS && (a.flags & FSM_FLAG_REMOVE_MEAN) && row == 0 && j == 0) nv[0] = csub(nv[0], a.dc[0]);
-#pragma unroll
-      for (int f = 0; f < CG; ++f) {
-        const int c = cg * CG + f;
-        nv[f] = cscale(nv[f], a.coef);
-        if (srcp) nv[f] = cadd(nv[f], srcp[((int64_t)(a.src_batch > 1 ? b : 0) * C + c) * S + sidx]);
-      }
+      for (int f = 0; f < CG; ++f) nv[f] = v[f][i];
+      axis0_nonlinear<NX, KIND, DIM>(a, nv, b, j0, row, cg);
     }
 #pragma unroll
     for (int f = 0; f < CG; ++f) {
       const int c = cg * CG + f;
       float2* up = state + ((int64_t)b * C + c) * S + sidx;
+      const int64_t toff = (tab_batch(a, b) * a.lin_ch + (a.lin_ch > 1 ? c : 0)) * S + sidx;
       float2 st;
-      if (!update) {
+      if (STG < 0) {
         st = *up;
+      } else if (INTEG == FSM_APPLY) {
+        st = cfma(tab[toff], *up, nv[f]);
+        *up = st;
       } else {
         float2* accp = aux + ((int64_t)b * a.n_aux * C + c) * S + sidx;
         float2* qp = aux + ((int64_t)b * a.n_aux * C + (a.n_aux > 1 ? C : 0) + c) * S + sidx;
-        const int64_t toff = (tab_batch(a, b) * a.lin_ch + (a.lin_ch > 1 ? c : 0)) * S + sidx;
-        if (STG >= 0)
-          st = etd_stage_c<INTEG, STG>(nv[f], up, accp, qp, tab + toff, a.ts);
-        else
-          st = etd_stage(a.integ, a.stage, nv[f], up, accp, qp, tab + toff, a.ts, (int64_t)C * S);
+        st = etd_stage_c<INTEG, STG>(nv[f], up, accp, qp, tab + toff, a.ts);
       }
-      if (a.slot >= 0 && (!update || last)) traj[(((int64_t)b * a.n_frames + a.slot) * C + c) * S + sidx] = st;
-      tileA[(f * W + col) * P + row] = cscale(st, pk.mask);
+      if (a.slot >= 0 && (STG < 0 || last)) traj[(((int64_t)b * a.n_frames + a.slot) * C + c) * S + sidx] = st;
+      v[f][i] = st;
     }
   }
 }
 
-// Axis-0 pass (2D: the column pass; 3D: the x pass). A CTA owns W adjacent
-// inner columns (contiguous in memory) of one sample, all NX rows:
+// The stage update of the other schemes, dispatched at run time: one rolled loop over the thread's
+// points, which pass through its own words of the shared buffer x (unrolled over registers the
+// dispatch would be repeated for every point).
+template <int NX, int KIND, int DIM>
+__device__ __forceinline__ void axis0_update_any(const StepArgs& a, float2 (&v)[RegKind<KIND, DIM>::CG][RegShape<NX>::E],
+                                                 float2* __restrict__ x, int b, int64_t j0, int t, int cg, bool last) {
+  using K = RegKind<KIND, DIM>;
+  constexpr int T = RegShape<NX>::T, E = RegShape<NX>::E, C = K::C, CG = K::CG;
+  const int64_t S = a.S, inner = S / NX;
+  // (a channel at a time would need the Leray projection's other channels: the group's go together)
+  float2* xs = x + threadIdx.x;
+#pragma unroll
+  for (int f = 0; f < CG; ++f)
+#pragma unroll
+    for (int i = 0; i < E; ++i) xs[(f * E + i) * 256] = v[f][i];
+#pragma unroll 1
+  for (int i = 0; i < E; ++i) {
+    const int row = t + T * i;
+    const int64_t sidx = (int64_t)row * inner + j0;
+    float2 nv[CG];
+#pragma unroll
+    for (int f = 0; f < CG; ++f) nv[f] = xs[(f * E + i) * 256];
+    axis0_nonlinear<NX, KIND, DIM>(a, nv, b, j0, row, cg);
+#pragma unroll
+    for (int f = 0; f < CG; ++f) {
+      const int c = cg * CG + f;
+      float2* accp = a.aux + ((int64_t)b * a.n_aux * C + c) * S + sidx;
+      float2* qp = a.aux + ((int64_t)b * a.n_aux * C + (a.n_aux > 1 ? C : 0) + c) * S + sidx;
+      const int64_t toff = (tab_batch(a, b) * a.lin_ch + (a.lin_ch > 1 ? c : 0)) * S + sidx;
+      const float2 st = etd_stage(a.integ, a.stage, nv[f], a.state + ((int64_t)b * C + c) * S + sidx, accp, qp,
+                                  a.tab + toff, a.ts, (int64_t)C * S);
+      if (a.slot >= 0 && last) a.traj[(((int64_t)b * a.n_frames + a.slot) * C + c) * S + sidx] = st;
+      xs[(f * E + i) * 256] = st;
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < CG; ++f)
+#pragma unroll
+    for (int i = 0; i < E; ++i) v[f][i] = xs[(f * E + i) * 256];
+}
+
+// Axis-0 pass (2D: the column pass; 3D: the x pass). A CTA owns W adjacent inner columns (contiguous
+// in memory) of one sample, all NX rows, a column's points in the registers of its T threads
+// throughout (col_fft):
 //   1. forward transform along axis 0 of the products -> N (+ Leray projection, + source)
 //   2. stage update at every point, recording when a step completes
 //   3. next stage field (mask, 1/N, i kx, streamfunction) -> inverse transform -> mid fields
-// Channels are processed in groups so that Convection needs one staging tile.
-// FAST: a SETDRK4 stage launch of a vorticity or convection program (channel groups of one
-// channel; the hoisted update, two CTAs per SM, k_axis0_r2); otherwise any scheme, the priming
-// launch included (k_axis0_r).
-// One channel group cg: a CTA of its own per group (grid.z), so that the channels of a velocity run
+// FAST: a SETDRK4 stage launch of a program with channel groups of one channel (the hoisted update,
+// k_axis0_r2); otherwise any scheme, the priming launch included (k_axis0_r). STG: the stage of a FAST launch where the kernel has one of its own
+// (-1: read from the arguments, the multi-plan kernels).
+// The code of a launch is kept small (one stage's update, one copy of the inverse transform).
+// One channel group cg: a CTA of its own per group, so that the channels of a velocity run
 // side by side instead of one after the other (3D Burgers 64^3 x 3: the x pass had 198 CTAs of three
 // channels each; with the kept columns of the 3D passes 7.03 -> 5.60 ms per 20 steps).
-template <int NX, int KIND, int DIM, bool FAST>
+// Bound: the latency of its rounds of loads (L2 hits: 6 of 12 cycles per issue at two CTAs per SM on
+// 256^2 x 34) and instruction issue. Against the staged tiles it replaced (products, update and each
+// field through shared tiles, tables loaded as used): vorticity 256^2 x 64 9.45 -> 8.68 ms per 50
+// steps, 512^2 x 5 6.86 -> 6.37 ms per 40, 3D Burgers 256^3 17.0 -> 14.3 ms per 4, 64^3 x 3 5.62 ->
+// 5.06 ms per 20.
+template <int NX, int KIND, int DIM, bool FAST, int STG = -1>
 __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, int cg) {
   using Cfg = ColCfg<NX>;
   using K = RegKind<KIND, DIM>;
-  constexpr int T = Cfg::T, E = Cfg::E, W = Cfg::W, P = Cfg::P, C = K::C, CG = K::CG;
+  constexpr int T = Cfg::T, E = Cfg::E, W = Cfg::W, C = K::C, CG = K::CG;
   extern __shared__ float2 smem[];
-  float2* twt = smem;                 // NX
-  float2* tileA = smem + NX;          // CG * W * P: products -> N -> next stage field
-  float2* tileB = tileA + CG * W * P; // W * P: transpose scratch and output staging
-  const int g = threadIdx.x / T, t = threadIdx.x % T;
+  float2* twt = smem;       // NX
+  float* kxs = (float*)(smem + NX);     // NX
+  float2* buf = smem + NX + NX / 2;     // two exchange buffers
+  int par = 0;
+  const int g = threadIdx.x % W, t = threadIdx.x / W;
   const int64_t c0 = (int64_t)tile * W;
-  const int64_t S = a.S;
-  const int64_t inner = S / NX;
+  const int64_t S = a.S, inner = S / NX;
+  const bool in = c0 + g < inner;
+  const int64_t j0 = in ? c0 + g : inner - 1;  // threads beyond the last column repeat it and store nothing
   load_reg_twiddles<NX>(twt, a.tw, threadIdx.x, 256);
+  for (int x = threadIdx.x; x < NX; x += 256) kxs[x] = a.kx[x];
   const bool last = a.stage == a.nstages - 1;
-  float kxr[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) kxr[j] = a.kx[t + T * j];
-  const int64_t gcol = c0 + g;
-  const PointK<DIM> gk = point_k<DIM>(a, 0, gcol < inner ? gcol : inner - 1);
 
+  float2 st[CG][E];
+  float2 o1[FAST ? E : 1];
   if (a.stage >= 0) {
+#pragma unroll
     for (int f = 0; f < CG; ++f) {
-      const float2* src = a.prod + ((int64_t)b * a.n_prod + cg * CG + f) * a.ms;
-      // all loads of the tile are issued before the shared-memory stores
-      float2 buf[NX * W / 256];
+      const float2* src = a.prod + ((int64_t)b * a.n_prod + cg * CG + f) * a.ms + j0;
 #pragma unroll
-      for (int it = 0; it < NX * W / 256; ++it) {
-        const int idx = threadIdx.x + it * 256;
-        const int row = idx / W, col = idx % W;
-        if (c0 + col < inner) buf[it] = src[(int64_t)row * a.wp + c0 + col];
-      }
+      for (int j = 0; j < E; ++j) st[f][j] = src[(int64_t)(t + T * j) * a.wp];
+    }
+    if constexpr (FAST) {
+      const float2* o = ((STG >= 0 ? STG : a.stage) <= 1 ? a.state + ((int64_t)b * C + cg) * S : a.aux + ((int64_t)b * a.n_aux * C + cg) * S) + j0;
 #pragma unroll
-      for (int it = 0; it < NX * W / 256; ++it) {
-        const int idx = threadIdx.x + it * 256;
-        const int row = idx / W, col = idx % W;
-        if (c0 + col < inner) tileA[(f * W + col) * P + row] = buf[it];
-      }
+      for (int j = 0; j < E; ++j) o1[j] = o[(int64_t)(t + T * j) * inner];
     }
-    __syncthreads();
-    for (int f = 0; f < CG; ++f) {
-      float2* colp = tileA + (f * W + g) * P;
-      float2 v[E];
+    __syncthreads();  // the twiddles and wavenumbers
 #pragma unroll
-      for (int j = 0; j < E; ++j) v[j] = colp[t + T * j];
-      reg_fft<NX, false>(v, tileB + g * P, twt, t);
-#pragma unroll
-      for (int j = 0; j < E; ++j) colp[t + T * j] = v[j];
-    }
-  }
-  __syncthreads();
-
-  if constexpr (FAST) {
-    switch (a.stage) {
-      case 0: axis0_update_hoisted<NX, KIND, DIM, 0>(a, tileA, b, c0, cg, last); break;
-      case 1: axis0_update_hoisted<NX, KIND, DIM, 1>(a, tileA, b, c0, cg, last); break;
-      case 2: axis0_update_hoisted<NX, KIND, DIM, 2>(a, tileA, b, c0, cg, last); break;
-      default: axis0_update_hoisted<NX, KIND, DIM, 3>(a, tileA, b, c0, cg, last); break;
-    }
-  } else if (a.stage >= 0 && a.integ == FSM_SETDRK4) {
-    switch (a.stage) {
-      case 0: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 0>(a, tileA, b, c0, cg, last); break;
-      case 1: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 1>(a, tileA, b, c0, cg, last); break;
-      case 2: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 2>(a, tileA, b, c0, cg, last); break;
-      default: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 3>(a, tileA, b, c0, cg, last); break;
-    }
+    for (int f = 0; f < CG; ++f) col_fft<NX, false>(st[f], buf, par, twt, t, g);
   } else {
-    axis0_update<NX, KIND, DIM, -1, -1>(a, tileA, b, c0, cg, last);
+    __syncthreads();
+  }
+  if (in) {
+    if constexpr (FAST && STG >= 0) {
+      axis0_update_hoisted<NX, KIND, DIM, (STG >= 0 ? STG : 0)>(a, st[0], o1, b, j0, t, cg, last);
+    } else if constexpr (FAST) {
+      switch (a.stage) {
+        case 0: axis0_update_hoisted<NX, KIND, DIM, 0>(a, st[0], o1, b, j0, t, cg, last); break;
+        case 1: axis0_update_hoisted<NX, KIND, DIM, 1>(a, st[0], o1, b, j0, t, cg, last); break;
+        case 2: axis0_update_hoisted<NX, KIND, DIM, 2>(a, st[0], o1, b, j0, t, cg, last); break;
+        default: axis0_update_hoisted<NX, KIND, DIM, 3>(a, st[0], o1, b, j0, t, cg, last); break;
+      }
+    } else if (CG > 1 && a.stage >= 0 && a.integ == FSM_SETDRK4) {
+      switch (a.stage) {
+        case 0: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 0>(a, st, b, j0, t, cg, last); break;
+        case 1: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 1>(a, st, b, j0, t, cg, last); break;
+        case 2: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 2>(a, st, b, j0, t, cg, last); break;
+        default: axis0_update<NX, KIND, DIM, FSM_SETDRK4, 3>(a, st, b, j0, t, cg, last); break;
+      }
+    } else if (a.stage < 0) {
+      axis0_update<NX, KIND, DIM, -1, -1>(a, st, b, j0, t, cg, last);
+    } else if (a.integ == FSM_APPLY) {
+      axis0_update<NX, KIND, DIM, FSM_APPLY, 0>(a, st, b, j0, t, cg, last);
+    } else {
+      // words of its own in a buffer of its own (behind the exchange buffers)
+      axis0_update_any<NX, KIND, DIM>(a, st, smem + Cfg::WORDS, b, j0, t, cg, last);
+    }
   }
   if (!a.emit) return;  // uniform
   // 2D: columns from hk on are dealiased and the row pass does not read them: nothing to store.
   // 3D: the next passes read the columns (jm, jl) with jm kept and jl < hk.
   if (DIM == 2 && c0 >= (int64_t)a.hk) return;  // uniform
+  bool live = in;
+  if (DIM == 2) live = j0 < (int64_t)a.hk && in;
+  else if (live) live = (int)(j0 % a.H) < a.hk && (a.hk == a.H || a.keepm[(int)(j0 / a.H)]);
   if (a.tile_zero && a.tile_zero[tile]) {
     if (DIM == 3 && a.hk < a.H) return;
-    // every column of this tile is dealiased: the next-stage fields are zero here, written
-    // directly (coalesced rows of W columns) without the transforms
+    // every column of this tile is dealiased: the next-stage fields are zero here
     constexpr int NMO = (KIND == FSM_NL_CONVECTION) ? 2 : K::NMG;  // fields of this channel group
     const int m0 = (KIND == FSM_NL_CONVECTION) ? cg * 2 : 0;
 #pragma unroll 1
     for (int mf = 0; mf < NMO; ++mf) {
-      float2* dst = a.mid + ((int64_t)b * a.n_mid + m0 + mf) * a.ms;
+      float2* dst = a.mid + ((int64_t)b * a.n_mid + m0 + mf) * a.ms + j0;
 #pragma unroll
-      for (int it = 0; it < NX * W / 256; ++it) {
-        const int idx = threadIdx.x + it * 256;
-        const int row = idx / W, cc = idx % W;
-        if (c0 + cc < inner) dst[(int64_t)row * a.wp + c0 + cc] = make_float2(0.f, 0.f);
-      }
+      for (int j = 0; j < E; ++j)
+        if (live) dst[(int64_t)(t + T * j) * a.wp] = make_float2(0.f, 0.f);
     }
     return;  // uniform across the CTA
   }
-  __syncthreads();
-  const int64_t sj = c0 + threadIdx.x % W;  // the column this thread stores
-  bool live = sj < inner;
-  if (DIM == 2) live = sj < (int64_t)a.hk;
-  else if (live) live = (int)(sj % a.H) < a.hk && (a.hk == a.H || a.keepm[(int)(sj / a.H)]);
-
-  // Next-stage fields: each group transforms its own column into tileB, then the CTA
-  // stores the tile with a coalesced mapping (rows of W adjacent columns).
-  for (int mf = 0; mf < K::NMG; ++mf) {
-    const int f = (KIND == FSM_NL_VORTICITY || KIND == FSM_NL_KS) ? 0 : (mf >> 1);
-    const float2* colp = tileA + (f * W + g) * P;
+  const PointK<DIM> gk = point_k<DIM>(a, 0, j0);
+  const uint8_t kc = (DIM == 2) ? a.keepy[j0] : (uint8_t)(a.keepm[(int)(j0 / a.H)] & a.keepy[(int)(j0 % a.H)]);
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    const int row = t + T * j;
+    const float m = (float)(a.keepx[row] & kc) * a.scale;
+#pragma unroll
+    for (int f = 0; f < CG; ++f) st[f][j] = cscale(st[f][j], m);
+  }
+  // (channel by channel for the Leray projection's groups: the fields of channel f are 2 f, 2 f + 1)
+#pragma unroll
+  for (int f = 0; f < CG; ++f) {
+#pragma unroll 1
+  for (int mf = f * 2; mf < (CG > 1 ? f * 2 + 2 : K::NMG); ++mf) {
     float2 v[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-      const float2 d = colp[t + T * j];
-      const float kxv = kxr[j];
-      float2 x;
+      // vorticity: 0: psi = -w/lap, 1: i kx psi, 2: w, 3: i kx w; KS: 0: phi, 1: i kx phi;
+      // velocity (per channel): u_c, i kx u_c
+      const float kxv = kxs[t + T * j];
+      float2 x = st[f][j];
       if (KIND == FSM_NL_VORTICITY) {
-        // 0: psi = -w/lap, 1: i kx psi, 2: w, 3: i kx w
-        if (mf < 2) {
-          const float lap = -(kxv * kxv + gk.ky * gk.ky);
-          // fast division: within 2 ulp for |lap| below 2^126, far above any mesh's 2 (pi NX / L)^2
-          const float il = (lap == 0.f) ? 1.f : __fdividef(1.f, lap);
-          const float2 psi = cscale(d, -il);
-          x = (mf == 0) ? psi : cscale(cmuli(psi), kxv);
-        } else {
-          x = (mf == 2) ? d : cscale(cmuli(d), kxv);
-        }
-      } else {
-        // KS: 0: phi, 1: i kx phi; convection (per channel): u_c, i kx u_c
-        x = (mf & 1) ? cscale(cmuli(d), kxv) : d;
+        const float lap = -(kxv * kxv + gk.ky * gk.ky);
+        // fast division: within 2 ulp for |lap| below 2^126, far above any mesh's 2 (pi NX / L)^2
+        const float il = (lap == 0.f) ? 1.f : __fdividef(1.f, lap);
+        x = cscale(x, mf < 2 ? -il : 1.f);
       }
-      v[j] = x;
+      const float2 ix = cscale(cmuli(x), kxv);
+      v[j] = (mf & 1) ? ix : x;
     }
-    float2* ob = tileB + g * P;
-    reg_fft<NX, true>(v, ob, twt, t);
-#pragma unroll
-    for (int j = 0; j < E; ++j) ob[t + T * j] = v[j];
-    __syncthreads();
+    col_fft<NX, true>(v, buf, par, twt, t, g);
     const int mout = (KIND == FSM_NL_CONVECTION) ? cg * 2 + mf : mf;
-    float2* dst = a.mid + ((int64_t)b * a.n_mid + mout) * a.ms;
+    float2* dst = a.mid + ((int64_t)b * a.n_mid + mout) * a.ms + j0;
+    if (live) {
 #pragma unroll
-    for (int it = 0; it < NX * W / 256; ++it) {
-      const int idx = threadIdx.x + it * 256;
-      const int row = idx / W, cc = idx % W;
-      if (live) dst[(int64_t)row * a.wp + c0 + cc] = tileB[cc * P + row];
+      for (int j = 0; j < E; ++j) dst[(int64_t)(t + T * j) * a.wp] = v[j];
     }
-    __syncthreads();
+  }
   }
 }
 
