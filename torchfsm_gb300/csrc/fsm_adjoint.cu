@@ -408,35 +408,34 @@ int fsm_step_adjoint(const FsmPlan* p, int32_t batch, const void* u, const void*
   const float al[4] = {0.f, 1.f, 1.f, 2.f}, be[4] = {0.f, 0.f, 0.f, -1.f};
   float2* outs[4] = {n0, n1, n2, n3};
   for (int s = 0; s < 4; ++s) {
-    k_adjs_fields<<<gh, 256, 0, st>>>(g, T, th, C, s > 0, xs[s], ys[s], al[s], zs[s], be[s], s == 1 ? a1 : nullptr, F);
-    if ((rc = cuda_check(cudaGetLastError(), "k_adjs_fields"))) return rc;
-    if ((rc = fsm_irfftn(p, nb * batch * C, F, P[s], stream))) return rc;
-    k_adjs_product<<<gr, 256, 0, st>>>(tr, C, p->R, p->nl_coef, P[s], Q);
-    if ((rc = cuda_check(cudaGetLastError(), "k_adjs_product"))) return rc;
-    if ((rc = fsm_rfftn(p, batch * C, Q, outs[s], stream))) return rc;
+    if ((rc = launch_pdl(false, k_adjs_fields, gh, 256, 0, st, "k_adjs_fields", g, T, th, C, (int)(s > 0), xs[s], ys[s],
+                         al[s], zs[s], be[s], s == 1 ? a1 : nullptr, F)))
+      return rc;
+    if ((rc = inverse_real(p, nb * batch * C, F, P[s], false, st))) return rc;
+    if ((rc = launch_pdl(false, k_adjs_product, gr, 256, 0, st, "k_adjs_product", tr, C, p->R, p->nl_coef, P[s], Q)))
+      return rc;
+    if ((rc = forward_real(p, batch * C, Q, outs[s], false, st))) return rc;
   }
 
   // backward
-  k_adjs_begin<<<gh, 256, 0, st>>>(T, th, C, (const float2*)ubar_next, uu, n0, n1, n2, n3, ubar_acc, n0b, n1b, n2b,
-                                   nbs, tbar);
-  if ((rc = cuda_check(cudaGetLastError(), "k_adjs_begin"))) return rc;
+  if ((rc = launch_pdl(false, k_adjs_begin, gh, 256, 0, st, "k_adjs_begin", T, th, C, (const float2*)ubar_next, uu, n0, n1,
+                       n2, n3, ubar_acc, n0b, n1b, n2b, nbs, tbar)))
+    return rc;
   AdjEnd e{F, uu, a1, n0, n1, n2, ubar_acc, a1b, n0b, n1b, n2b, nbs, (float2*)ubar, tbar};
   const float scale = p->nl_coef * (float)p->R;
   for (int s = 3; s >= 0; --s) {
     // w = coef N irfft(nbar); ubar_c = sum_c' w_c' d_c u_c', u_i w_c -> rfft -> combination
-    if ((rc = fsm_irfftn(p, batch * C, nbs, nbp, stream))) return rc;
+    if ((rc = inverse_real(p, batch * C, nbs, nbp, false, st))) return rc;
     const float* Ps = P[s];
     const float* g1 = nd > 1 ? Ps + 2 * tr : nullptr;
     const float* g2 = nd > 2 ? Ps + 3 * tr : nullptr;
-    switch (nd) {
-      case 1: k_adj_vjp_products<1><<<gr / C + 1, 256, 0, st>>>(batch, p->R, scale, nbp, Ps, Ps + tr, g1, g2, Q, Q + tr); break;
-      case 2: k_adj_vjp_products<2><<<gr / C + 1, 256, 0, st>>>(batch, p->R, scale, nbp, Ps, Ps + tr, g1, g2, Q, Q + tr); break;
-      default: k_adj_vjp_products<3><<<gr / C + 1, 256, 0, st>>>(batch, p->R, scale, nbp, Ps, Ps + tr, g1, g2, Q, Q + tr); break;
-    }
-    if ((rc = cuda_check(cudaGetLastError(), "k_adj_vjp_products"))) return rc;
-    if ((rc = fsm_rfftn(p, nb * batch * C, Q, F, stream))) return rc;
-    k_adjs_end<<<gh, 256, 0, st>>>(g, T, th, C, (float)(1.0 / (double)p->R), s, e);
-    if ((rc = cuda_check(cudaGetLastError(), "k_adjs_end"))) return rc;
+    const auto vjp = nd == 1 ? k_adj_vjp_products<1> : nd == 2 ? k_adj_vjp_products<2> : k_adj_vjp_products<3>;
+    if ((rc = launch_pdl(false, vjp, gr / C + 1, 256, 0, st, "k_adj_vjp_products", batch, p->R, scale, nbp, Ps, Ps + tr, g1,
+                         g2, Q, Q + tr)))
+      return rc;
+    if ((rc = forward_real(p, nb * batch * C, Q, F, false, st))) return rc;
+    if ((rc = launch_pdl(false, k_adjs_end, gh, 256, 0, st, "k_adjs_end", g, T, th, C, (float)(1.0 / (double)p->R), s, e)))
+      return rc;
   }
   return FSM_OK;
 }

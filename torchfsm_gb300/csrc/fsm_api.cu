@@ -702,6 +702,7 @@ size_t integrate_workspace_bytes(const FsmPlan* p, int32_t batch, int32_t steps)
 }  // namespace fsm
 
 namespace fsm {
+bool short_grid(const FsmPlan* p, int64_t fields);
 // Batches at or above kSplitPoints spectral points run in parts of about kPartPoints points
 // (2 to kMaxParts parts, at most one per sample) on as many streams. Measured on 256^2 x 64
 // (2.1 M points): one sequence 322 us per step, 2 parts 284, 4 parts 270, 8 parts 261.
@@ -987,6 +988,7 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   const int NP = (!allow_split || prof || cap != cudaStreamCaptureStatusNone) ? 1 : fsm::split_parts(p, batch);
   const bool split = NP > 1;
   if (!split) {
+    a.pdl = short_grid(p, (int64_t)batch * p->C);
     PlaneSequence q{p, batch_arrays(p, a, arr, 0, batch), record_slot, steps, st, prof};
     if ((rc = q.prime())) return rc;
     for (int k = 0; k < steps; ++k)
@@ -1041,6 +1043,52 @@ int integrate_with_workspace(const FsmPlan* p, int32_t batch, void* state, int32
 }
 }  // namespace fsm
 
+namespace fsm {
+// Whether a pass over `fields` fields is short enough for its tail and the next one's start to
+// matter (launch_pdl): up to 2 M spectral points. 3D Burgers 64^3 x 3 (1.2 M points): 5.03 -> 4.39 ms
+// per 20 steps; 256^3 (25 M): 14.3 -> 15.2 ms per 4, so longer passes launch plainly, as do the
+// adjoint step's kernels in their captured graph (22.2 -> 23.2 ms per iteration of 128^2 x 16).
+bool short_grid(const FsmPlan* p, int64_t fields) { return fields * p->S <= ((int64_t)1 << 21); }
+
+int forward_real(const FsmPlan* p, int64_t count, const float* in, float2* out, bool pdl, cudaStream_t st) {
+  if (count == 0) return FSM_OK;
+  const int nd = p->ndim;
+  const int nl = p->n[nd - 1];
+  int64_t rows = count * (p->R / nl);
+  int rc = transform_r2c_last(nl, in, out, rows, p->tw, pdl, st);
+  if (rc) return rc;
+  // outer axes, innermost first
+  int64_t inner = p->h;
+  for (int ax = nd - 2; ax >= 0; --ax) {
+    int64_t outer = count;
+    for (int j = 0; j < ax; ++j) outer *= p->n[j];
+    if (outer > 65535) return set_error(FSM_ERR_UNSUPPORTED, "rfftn: too many fields in one call");
+    rc = transform_c2c_strided(p->n[ax], false, out, outer, inner, p->tw, pdl, st);
+    if (rc) return rc;
+    inner *= p->n[ax];
+  }
+  return FSM_OK;
+}
+
+int inverse_real(const FsmPlan* p, int64_t count, float2* in, float* out, bool pdl, cudaStream_t st) {
+  if (count == 0) return FSM_OK;
+  const int nd = p->ndim;
+  int rc;
+  int64_t inner = p->h;
+  for (int ax = nd - 2; ax >= 0; --ax) {
+    int64_t outer = count;
+    for (int j = 0; j < ax; ++j) outer *= p->n[j];
+    if (outer > 65535) return set_error(FSM_ERR_UNSUPPORTED, "irfftn: too many fields in one call");
+    rc = transform_c2c_strided(p->n[ax], true, in, outer, inner, p->tw, pdl, st);
+    if (rc) return rc;
+    inner *= p->n[ax];
+  }
+  const int nl = p->n[nd - 1];
+  const int64_t rows = count * (p->R / nl);
+  return transform_c2r_last(nl, in, out, rows, (float)(1.0 / (double)p->R), p->tw, pdl, st);
+}
+}  // namespace fsm
+
 extern "C" {
 
 int fsm_integrate(const FsmPlan* p, int32_t batch, void* state, int32_t steps, const int32_t* record_slot, void* traj,
@@ -1065,44 +1113,12 @@ int fsm_integrate_profiled(const FsmPlan* p, int32_t batch, void* state, int32_t
 
 int fsm_rfftn(const FsmPlan* p, int32_t count, const float* in, void* out, void* stream) {
   if (!p || !in || !out || count < 0) return set_error(FSM_ERR_INVALID, "rfftn arguments");
-  if (count == 0) return FSM_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int nd = p->ndim;
-  const int nl = p->n[nd - 1];
-  int64_t rows = (int64_t)count * (p->R / nl);
-  int rc = transform_r2c_last(nl, in, (float2*)out, rows, p->tw, st);
-  if (rc) return rc;
-  // outer axes, innermost first
-  int64_t inner = p->h;
-  for (int ax = nd - 2; ax >= 0; --ax) {
-    int64_t outer = count;
-    for (int j = 0; j < ax; ++j) outer *= p->n[j];
-    if (outer > 65535) return set_error(FSM_ERR_UNSUPPORTED, "rfftn: too many fields in one call");
-    rc = transform_c2c_strided(p->n[ax], false, (float2*)out, outer, inner, p->tw, st);
-    if (rc) return rc;
-    inner *= p->n[ax];
-  }
-  return FSM_OK;
+  return fsm::forward_real(p, count, in, (float2*)out, fsm::short_grid(p, count), (cudaStream_t)stream);
 }
 
 int fsm_irfftn(const FsmPlan* p, int32_t count, void* in, float* out, void* stream) {
   if (!p || !in || !out || count < 0) return set_error(FSM_ERR_INVALID, "irfftn arguments");
-  if (count == 0) return FSM_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int nd = p->ndim;
-  int rc;
-  int64_t inner = p->h;
-  for (int ax = nd - 2; ax >= 0; --ax) {
-    int64_t outer = count;
-    for (int j = 0; j < ax; ++j) outer *= p->n[j];
-    if (outer > 65535) return set_error(FSM_ERR_UNSUPPORTED, "irfftn: too many fields in one call");
-    rc = transform_c2c_strided(p->n[ax], true, (float2*)in, outer, inner, p->tw, st);
-    if (rc) return rc;
-    inner *= p->n[ax];
-  }
-  const int nl = p->n[nd - 1];
-  const int64_t rows = (int64_t)count * (p->R / nl);
-  return transform_c2r_last(nl, (const float2*)in, out, rows, (float)(1.0 / (double)p->R), p->tw, st);
+  return fsm::inverse_real(p, count, (float2*)in, out, fsm::short_grid(p, count), (cudaStream_t)stream);
 }
 
 int fsm_nonfinite_flags(const FsmPlan* p, int32_t count, const void* fields, int32_t* flags, void* stream) {

@@ -60,6 +60,13 @@ __device__ __forceinline__ float2 cfma(float2 c, float2 b, float2 a) {
   return make_float2(fmaf(c.x, b.x, fmaf(-c.y, b.y, a.x)), fmaf(c.x, b.y, fmaf(c.y, b.x, a.y)));
 }
 
+// Programmatic dependent launch (launch_pdl): let the next grid in the stream be placed, and wait for
+// the grid before this one; both do nothing in a plain launch.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <bool INV>
 __device__ __forceinline__ void dft2(float2* v) {
   float2 a = v[0], b = v[1];

@@ -46,6 +46,7 @@ struct StepArgs {
   int hk;                     // last-axis columns of the stage fields stored and read (FsmPlan::hk)
   int64_t wp, ms;             // row pitch and field stride of mid / prod (FsmPlan::wp, ms)
   const int32_t* tab_entry;   // per sample: its coefficient-table entry (serving), or null
+  int pdl;                    // host: launch the passes as programmatic dependents (launch_pdl)
 };
 
 // The coefficient-table entry of sample b: its own entry from tab_entry when given (a serving
@@ -58,11 +59,14 @@ __device__ __forceinline__ int64_t tab_batch(const StepArgs& a, int b) {
 // without recording (fsm_api.cu).
 StepArgs base_args(const FsmPlan* p, void* state, int32_t batch, int32_t steps);
 
-int transform_r2c_last(int n, const float* in, float2* out, int64_t rows, const float2* tw, cudaStream_t st);
-int transform_c2r_last(int n, const float2* in, float* out, int64_t rows, float scale, const float2* tw,
+int transform_r2c_last(int n, const float* in, float2* out, int64_t rows, const float2* tw, bool pdl, cudaStream_t st);
+int transform_c2r_last(int n, const float2* in, float* out, int64_t rows, float scale, const float2* tw, bool pdl,
                        cudaStream_t st);
-int transform_c2c_strided(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw,
+int transform_c2c_strided(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw, bool pdl,
                           cudaStream_t st);
+// The whole real transforms of `count` fields (fsm_rfftn, fsm_irfftn), as programmatic dependents or plain launches.
+int forward_real(const FsmPlan* p, int64_t count, const float* in, float2* out, bool pdl, cudaStream_t st);
+int inverse_real(const FsmPlan* p, int64_t count, float2* in, float* out, bool pdl, cudaStream_t st);
 int launch_nonfinite(const float2* f, int64_t count, int64_t S, int32_t* flags, cudaStream_t st);
 
 // fsm_integrate without recording on a caller-provided workspace (fsm_api.cu).
@@ -133,6 +137,28 @@ struct ResConfig {
 bool resident_config(const FsmPlan* p, int batch, ResConfig* out);
 // a.steps steps of a.B samples in one launch, frames at a.slots (device) when given.
 int launch_resident(const FsmPlan* p, const ResConfig& c, const StepArgs& a, cudaStream_t st);
+
+// Programmatic dependent launch: the grid may start (its blocks are placed, constants are loaded)
+// while the one before it in the stream still runs; the kernel waits in pdl_wait() before it touches
+// anything that grid wrote or still reads. Every kernel launched this way calls pdl_wait() in every
+// thread before its first access to global memory other than the plan's twiddles and wavenumbers.
+// For chains of short kernels (short_grid, fsm_api.cu); not used for the parts
+// of a split batch, whose waiting blocks would take the places of other parts' running ones.
+template <class... P, class... A>
+inline int launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      const char* what, A&&... args) {
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.gridDim = grid;
+  lc.blockDim = block;
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  lc.attrs = &at;
+  lc.numAttrs = pdl ? 1 : 0;
+  return cuda_check(cudaLaunchKernelEx(&lc, kernel, P(args)...), what);
+}
 
 // Raise a kernel's dynamic shared-memory limit when it needs more than 48 KB. The
 // attribute is per function and per device; the size set is remembered per

@@ -16,6 +16,7 @@ int launch_plane_col(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
 // Batch mean of the k = 0 product (KS mean removal): dc = (1/B) sum_b sum_x prod[b][0][x][0..0],
 // the products being transformed along every axis but the first.
 __global__ void k_ks_mean(StepArgs a, int nx) {
+  pdl_wait();
   float acc = 0.f;
   const int total = a.B * nx;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
@@ -33,8 +34,7 @@ __global__ void k_ks_mean(StepArgs a, int nx) {
 }
 
 int launch_ks_mean(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
-  k_ks_mean<<<1, 256, 0, st>>>(a, p->n[0]);
-  return cuda_check(cudaGetLastError(), "k_ks_mean");
+  return launch_pdl(a.pdl, k_ks_mean, 1, 256, 0, st, "k_ks_mean", a, p->n[0]);
 }
 
 }  // namespace fsm

@@ -32,13 +32,11 @@ static int launch_axis0_r_mode(const StepArgs& a, cudaStream_t st) {
   if constexpr (STG >= 0) {
     int rc = prep_smem(k_axis0_r2<NX, KIND, DIM, STG>, smem);
     if (rc) return rc;
-    k_axis0_r2<NX, KIND, DIM, STG><<<grid, 256, smem, st>>>(a);
-    return cuda_check(cudaGetLastError(), "k_axis0_r2");
+    return launch_pdl(a.pdl, k_axis0_r2<NX, KIND, DIM, STG>, grid, 256, smem, st, "k_axis0_r2", a);
   } else {
     int rc = prep_smem(k_axis0_r<NX, KIND, DIM>, smem);
     if (rc) return rc;
-    k_axis0_r<NX, KIND, DIM><<<grid, 256, smem, st>>>(a);
-    return cuda_check(cudaGetLastError(), "k_axis0_r");
+    return launch_pdl(a.pdl, k_axis0_r<NX, KIND, DIM>, grid, 256, smem, st, "k_axis0_r", a);
   }
 }
 

@@ -251,7 +251,7 @@ __device__ __forceinline__ void axis0_update_hoisted(const StepArgs& a, float2 (
   const float2* __restrict__ o2p = (STG == 1) ? accp : qp;
   // The operands of HALF points are loaded in one batch (one round of memory latency each half). The
   // SETDRK coefficients are real (k_phi_tables): only the exponentials are read as complex.
-  constexpr int HALF = E > 8 ? 8 : E;
+  constexpr int HALF = E > 8 ? (DIM == 2 && STG <= 1 ? 4 : 8) : E;
 #pragma unroll
   for (int h0 = 0; h0 < E; h0 += HALF) {
     float2 o2[HALF], em[HALF], e2[HALF];
@@ -431,6 +431,7 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, i
   const int64_t j0 = in ? c0 + g : inner - 1;  // threads beyond the last column repeat it and store nothing
   load_reg_twiddles<NX>(twt, a.tw, threadIdx.x, 256);
   for (int x = threadIdx.x; x < NX; x += 256) kxs[x] = a.kx[x];
+  pdl_wait();
   const bool last = a.stage == a.nstages - 1;
 
   float2 st[CG][E];
@@ -597,6 +598,7 @@ __device__ __forceinline__ void plane_row_body(const StepArgs& a, int blk, int b
   const int groups = blockDim.x / T;
   float2* scr = smem + NY + g * SCR;
   load_reg_twiddles<NY>(twt, a.tw, threadIdx.x, blockDim.x);
+  pdl_wait();
   __syncthreads();
   const int r0 = (blk * groups + g) * 2;
   const int64_t S = a.ms;  // field stride of the stage fields and products

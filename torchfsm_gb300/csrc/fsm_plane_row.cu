@@ -20,8 +20,7 @@ static int launch_row_r_hk(int nx, const StepArgs& a, cudaStream_t st) {
   int rc = prep_smem(k_plane_row_r<NY, KIND, HK>, smem);
   if (rc) return rc;
   dim3 grid(groups_needed / groups, a.B);
-  k_plane_row_r<NY, KIND, HK><<<grid, threads, smem, st>>>(a);
-  return cuda_check(cudaGetLastError(), "k_plane_row_r");
+  return launch_pdl(a.pdl, k_plane_row_r<NY, KIND, HK>, grid, threads, smem, st, "k_plane_row_r", a);
 }
 
 // The 2/3 rule's stored prefix (NY/3 + 1 columns) or every column.

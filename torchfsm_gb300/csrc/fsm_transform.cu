@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_r2c_last(const float* __
   const int t = threadIdx.x % Cfg::G;
   float2* z = smem + N + g * N;
   load_twiddles(tw, master, kTwiddleMax, N, threadIdx.x, Cfg::THREADS);
+  pdl_wait();
   const int64_t r0 = ((int64_t)blockIdx.x * Cfg::GROUPS + g) * 2;
   const bool has0 = r0 < rows, has1 = r0 + 1 < rows;
   for (int n = t; n < N; n += Cfg::G) {
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_c2r_last(const float2* _
   const int t = threadIdx.x % Cfg::G;
   float2* z = smem + N + g * N;
   load_twiddles(tw, master, kTwiddleMax, N, threadIdx.x, Cfg::THREADS);
+  pdl_wait();
   const int64_t r0 = ((int64_t)blockIdx.x * Cfg::GROUPS + g) * 2;
   const bool has0 = r0 < rows, has1 = r0 + 1 < rows;
   for (int k = t; k < H; k += Cfg::G) {
@@ -81,54 +83,53 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_c2r_last(const float2* _
 }
 
 template <int N>
-static int launch_r2c(const float* in, float2* out, int64_t rows, const float2* tw, cudaStream_t st) {
+static int launch_r2c(const float* in, float2* out, int64_t rows, const float2* tw, bool pdl, cudaStream_t st) {
   using Cfg = RowCfg<N>;
   int rc = prep_smem(k_r2c_last<N>, Cfg::SMEM);
   if (rc) return rc;
   const int64_t pairs = (rows + 1) / 2;
   const int64_t blocks = (pairs + Cfg::GROUPS - 1) / Cfg::GROUPS;
-  k_r2c_last<N><<<(unsigned)blocks, Cfg::THREADS, Cfg::SMEM, st>>>(in, out, rows, tw);
-  return cuda_check(cudaGetLastError(), "k_r2c_last");
+  return launch_pdl(pdl, k_r2c_last<N>, (unsigned)blocks, Cfg::THREADS, Cfg::SMEM, st, "k_r2c_last", in, out, rows, tw);
 }
 
 template <int N>
-static int launch_c2r(const float2* in, float* out, int64_t rows, float scale, const float2* tw, cudaStream_t st) {
+static int launch_c2r(const float2* in, float* out, int64_t rows, float scale, const float2* tw, bool pdl, cudaStream_t st) {
   using Cfg = RowCfg<N>;
   int rc = prep_smem(k_c2r_last<N>, Cfg::SMEM);
   if (rc) return rc;
   const int64_t pairs = (rows + 1) / 2;
   const int64_t blocks = (pairs + Cfg::GROUPS - 1) / Cfg::GROUPS;
-  k_c2r_last<N><<<(unsigned)blocks, Cfg::THREADS, Cfg::SMEM, st>>>(in, out, rows, scale, tw);
-  return cuda_check(cudaGetLastError(), "k_c2r_last");
+  return launch_pdl(pdl, k_c2r_last<N>, (unsigned)blocks, Cfg::THREADS, Cfg::SMEM, st, "k_c2r_last", in, out, rows,
+                    scale, tw);
 }
 
-int transform_r2c_last(int n, const float* in, float2* out, int64_t rows, const float2* tw, cudaStream_t st) {
+int transform_r2c_last(int n, const float* in, float2* out, int64_t rows, const float2* tw, bool pdl, cudaStream_t st) {
   switch (n) {
-    case 16: return launch_r2c<16>(in, out, rows, tw, st);
-    case 32: return launch_r2c<32>(in, out, rows, tw, st);
-    case 64: return launch_r2c<64>(in, out, rows, tw, st);
-    case 128: return launch_r2c<128>(in, out, rows, tw, st);
-    case 256: return launch_r2c<256>(in, out, rows, tw, st);
-    case 512: return launch_r2c<512>(in, out, rows, tw, st);
-    case 1024: return launch_r2c<1024>(in, out, rows, tw, st);
-    case 2048: return launch_r2c<2048>(in, out, rows, tw, st);
-    case 4096: return launch_r2c<4096>(in, out, rows, tw, st);
+    case 16: return launch_r2c<16>(in, out, rows, tw, pdl, st);
+    case 32: return launch_r2c<32>(in, out, rows, tw, pdl, st);
+    case 64: return launch_r2c<64>(in, out, rows, tw, pdl, st);
+    case 128: return launch_r2c<128>(in, out, rows, tw, pdl, st);
+    case 256: return launch_r2c<256>(in, out, rows, tw, pdl, st);
+    case 512: return launch_r2c<512>(in, out, rows, tw, pdl, st);
+    case 1024: return launch_r2c<1024>(in, out, rows, tw, pdl, st);
+    case 2048: return launch_r2c<2048>(in, out, rows, tw, pdl, st);
+    case 4096: return launch_r2c<4096>(in, out, rows, tw, pdl, st);
   }
   return set_error(FSM_ERR_UNSUPPORTED, "r2c: unsupported length " + std::to_string(n));
 }
 
 int transform_c2r_last(int n, const float2* in, float* out, int64_t rows, float scale, const float2* tw,
-                       cudaStream_t st) {
+                       bool pdl, cudaStream_t st) {
   switch (n) {
-    case 16: return launch_c2r<16>(in, out, rows, scale, tw, st);
-    case 32: return launch_c2r<32>(in, out, rows, scale, tw, st);
-    case 64: return launch_c2r<64>(in, out, rows, scale, tw, st);
-    case 128: return launch_c2r<128>(in, out, rows, scale, tw, st);
-    case 256: return launch_c2r<256>(in, out, rows, scale, tw, st);
-    case 512: return launch_c2r<512>(in, out, rows, scale, tw, st);
-    case 1024: return launch_c2r<1024>(in, out, rows, scale, tw, st);
-    case 2048: return launch_c2r<2048>(in, out, rows, scale, tw, st);
-    case 4096: return launch_c2r<4096>(in, out, rows, scale, tw, st);
+    case 16: return launch_c2r<16>(in, out, rows, scale, tw, pdl, st);
+    case 32: return launch_c2r<32>(in, out, rows, scale, tw, pdl, st);
+    case 64: return launch_c2r<64>(in, out, rows, scale, tw, pdl, st);
+    case 128: return launch_c2r<128>(in, out, rows, scale, tw, pdl, st);
+    case 256: return launch_c2r<256>(in, out, rows, scale, tw, pdl, st);
+    case 512: return launch_c2r<512>(in, out, rows, scale, tw, pdl, st);
+    case 1024: return launch_c2r<1024>(in, out, rows, scale, tw, pdl, st);
+    case 2048: return launch_c2r<2048>(in, out, rows, scale, tw, pdl, st);
+    case 4096: return launch_c2r<4096>(in, out, rows, scale, tw, pdl, st);
   }
   return set_error(FSM_ERR_UNSUPPORTED, "c2r: unsupported length " + std::to_string(n));
 }

@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(256) k_c2c_strided_r(float2* __restrict__ data
   const int64_t c0 = (int64_t)blockIdx.x * W;
   float2* base = data + (int64_t)blockIdx.y * N * inner;
   load_reg_twiddles<N>(twt, master, threadIdx.x, 256);
+  pdl_wait();
   {
     float2 buf[N * W / 256];
 #pragma unroll
@@ -69,23 +70,22 @@ __global__ void __launch_bounds__(256) k_c2c_strided_r(float2* __restrict__ data
 }
 
 template <int N, bool INV>
-static int launch_c2c_r(float2* data, int64_t outer, int64_t inner, const float2* tw, cudaStream_t st) {
+static int launch_c2c_r(float2* data, int64_t outer, int64_t inner, const float2* tw, bool pdl, cudaStream_t st) {
   using Cfg = TileCfg<N>;
   const size_t smem = (size_t)(N + 2 * Cfg::W * Cfg::P) * sizeof(float2);
   int rc = prep_smem(k_c2c_strided_r<N, INV>, smem);
   if (rc) return rc;
   if (outer > 65535) return set_error(FSM_ERR_UNSUPPORTED, "c2c: too many transforms in one launch");
   dim3 grid((unsigned)((inner + Cfg::W - 1) / Cfg::W), (unsigned)outer);
-  k_c2c_strided_r<N, INV><<<grid, 256, smem, st>>>(data, inner, tw);
-  return cuda_check(cudaGetLastError(), "k_c2c_strided_r");
+  return launch_pdl(pdl, k_c2c_strided_r<N, INV>, grid, 256, smem, st, "k_c2c_strided_r", data, inner, tw);
 }
 
-int transform_c2c_strided(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw,
-                              cudaStream_t st) {
+int transform_c2c_strided(int n, bool inverse, float2* data, int64_t outer, int64_t inner, const float2* tw, bool pdl,
+                          cudaStream_t st) {
 #define FSM_C2CR_CASE(NN)                                                                    \
   case NN:                                                                                   \
-    return inverse ? launch_c2c_r<NN, true>(data, outer, inner, tw, st)                      \
-                   : launch_c2c_r<NN, false>(data, outer, inner, tw, st);
+    return inverse ? launch_c2c_r<NN, true>(data, outer, inner, tw, pdl, st)                      \
+                   : launch_c2c_r<NN, false>(data, outer, inner, tw, pdl, st);
   switch (n) {
     FSM_C2CR_CASE(16)
     FSM_C2CR_CASE(32)
@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(256) k_axis1_inv_r(StepArgs a) {
   const int64_t plane = (int64_t)NY * H;
   const int64_t S = a.S;
   load_reg_twiddles<NY>(twt, a.tw, threadIdx.x, 256);
+  pdl_wait();
   const float2* in0 = a.mid + ((int64_t)b * a.n_mid + 2 * c) * S + (int64_t)x * plane;
   const float2* in1 = in0 + S;
   {
@@ -254,6 +255,7 @@ __global__ void __launch_bounds__(256, 2) k_axis2_r(StepArgs a) {
   float2* scr = smem + NZ + g * SCR;
   float* ust = (float*)(smem + NZ + groups * SCR) + (size_t)g * 3 * NZ;  // u0, u1, u2 of the group's row
   load_reg_twiddles<NZ>(twt, a.tw, threadIdx.x, blockDim.x);
+  pdl_wait();
   __syncthreads();
   const int b = blockIdx.y;
   const int64_t S = a.S;
@@ -338,8 +340,7 @@ static int launch_axis1_inv(int n0, const StepArgs& a, cudaStream_t st) {
   int rc = prep_smem(k_axis1_inv_r<NY>, smem);
   if (rc) return rc;
   dim3 grid((unsigned)((a.hk + Cfg::W - 1) / Cfg::W), (unsigned)n0, (unsigned)(a.B * (a.n_mid / 2)));
-  k_axis1_inv_r<NY><<<grid, 256, smem, st>>>(a);
-  return cuda_check(cudaGetLastError(), "k_axis1_inv_r");
+  return launch_pdl(a.pdl, k_axis1_inv_r<NY>, grid, 256, smem, st, "k_axis1_inv_r", a);
 }
 
 template <int NZ, int KIND, int HK>
@@ -354,8 +355,7 @@ static int launch_axis2_hk(const StepArgs& a, cudaStream_t st) {
   int rc = prep_smem(k_axis2_r<NZ, KIND, HK>, smem);
   if (rc) return rc;
   dim3 grid((unsigned)((groups_needed + groups - 1) / groups), a.B);
-  k_axis2_r<NZ, KIND, HK><<<grid, threads, smem, st>>>(a);
-  return cuda_check(cudaGetLastError(), "k_axis2_r");
+  return launch_pdl(a.pdl, k_axis2_r<NZ, KIND, HK>, grid, threads, smem, st, "k_axis2_r", a);
 }
 
 // The 2/3 rule's prefix (NZ/3 + 1 columns) or every column.
@@ -394,7 +394,8 @@ int launch_volume_axis2(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
 }
 
 int launch_volume_axis1_fwd(const FsmPlan* p, const StepArgs& a, cudaStream_t st) {
-  return transform_c2c_strided(p->n[1], false, a.prod, (int64_t)a.B * a.n_prod * p->n[0], a.H, p->tw, st);
+  return transform_c2c_strided(p->n[1], false, a.prod, (int64_t)a.B * a.n_prod * p->n[0], a.H, p->tw, a.pdl != 0,
+                               st);
 }
 
 }  // namespace fsm
