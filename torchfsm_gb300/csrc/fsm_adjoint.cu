@@ -23,6 +23,13 @@ __global__ void k_adj_vjp_products(int B, int64_t R, float scale, const float* _
                                    const float* __restrict__ u, const float* __restrict__ g0,
                                    const float* __restrict__ g1, const float* __restrict__ g2,
                                    float* __restrict__ ubar, float* __restrict__ uw) {
+  fsm::pdl_wait();
+  nbar = fsm::pdl_ptr(nbar);
+  u = fsm::pdl_ptr(u);
+  g0 = fsm::pdl_ptr(g0);
+  g1 = fsm::pdl_ptr(g1);
+  g2 = fsm::pdl_ptr(g2);
+  fsm::pdl_trigger();
   constexpr int C = ND;
   const float* g[3] = {g0, g1, g2};
   const int64_t total = (int64_t)B * R;
@@ -196,6 +203,11 @@ __device__ __forceinline__ float2 xe(float2 a, float em1) { return make_float2(f
 __global__ void k_adjs_fields(AdjGeom g, AdjTabs T, int64_t total, int C, int combine, const float2* __restrict__ x,
                               const float2* __restrict__ y, float alpha, const float2* __restrict__ z, float beta,
                               float2* __restrict__ store, float2* __restrict__ F) {
+  fsm::pdl_wait();
+  x = fsm::pdl_ptr(x);
+  y = fsm::pdl_ptr(y);
+  z = fsm::pdl_ptr(z);
+  fsm::pdl_trigger();
   const int64_t S = T.S;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = q % S;
@@ -219,6 +231,9 @@ __global__ void k_adjs_fields(AdjGeom g, AdjTabs T, int64_t total, int C, int co
 // p[b][c][r] = coef sum_i u_i g_i[c] with u_i = P[0][b][i][r], g_i[c] = P[1 + i][b][c][r].
 __global__ void k_adjs_product(int64_t total, int C, int64_t R, float coef, const float* __restrict__ P,
                                float* __restrict__ p) {
+  fsm::pdl_wait();
+  P = fsm::pdl_ptr(P);
+  fsm::pdl_trigger();
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = q % R;
     const int64_t b = q / ((int64_t)C * R);
@@ -236,6 +251,15 @@ __global__ void k_adjs_begin(AdjTabs T, int64_t total, int C, const float2* __re
                              const float2* __restrict__ n2, const float2* __restrict__ n3, float2* __restrict__ ubar,
                              float2* __restrict__ n0b, float2* __restrict__ n1b, float2* __restrict__ n2b,
                              float2* __restrict__ nbs, double* __restrict__ tb) {
+  fsm::pdl_wait();
+  ub = fsm::pdl_ptr(ub);
+  u = fsm::pdl_ptr(u);
+  n0 = fsm::pdl_ptr(n0);
+  n1 = fsm::pdl_ptr(n1);
+  n2 = fsm::pdl_ptr(n2);
+  n3 = fsm::pdl_ptr(n3);
+  tb = fsm::pdl_ptr(tb);
+  fsm::pdl_trigger();
   const int64_t S = T.S;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = q % S;
@@ -271,6 +295,8 @@ struct AdjEnd {
 };
 
 __global__ void k_adjs_end(AdjGeom g, AdjTabs T, int64_t total, int C, float inv_n, int mode, AdjEnd e) {
+  fsm::pdl_wait();
+  fsm::pdl_trigger();
   const int64_t S = T.S;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = q % S;
@@ -408,33 +434,33 @@ int fsm_step_adjoint(const FsmPlan* p, int32_t batch, const void* u, const void*
   const float al[4] = {0.f, 1.f, 1.f, 2.f}, be[4] = {0.f, 0.f, 0.f, -1.f};
   float2* outs[4] = {n0, n1, n2, n3};
   for (int s = 0; s < 4; ++s) {
-    if ((rc = launch_pdl(false, k_adjs_fields, gh, 256, 0, st, "k_adjs_fields", g, T, th, C, (int)(s > 0), xs[s], ys[s],
+    if ((rc = launch_pdl(true, k_adjs_fields, gh, 256, 0, st, "k_adjs_fields", g, T, th, C, (int)(s > 0), xs[s], ys[s],
                          al[s], zs[s], be[s], s == 1 ? a1 : nullptr, F)))
       return rc;
-    if ((rc = inverse_real(p, nb * batch * C, F, P[s], false, st))) return rc;
-    if ((rc = launch_pdl(false, k_adjs_product, gr, 256, 0, st, "k_adjs_product", tr, C, p->R, p->nl_coef, P[s], Q)))
+    if ((rc = inverse_real(p, nb * batch * C, F, P[s], true, st))) return rc;
+    if ((rc = launch_pdl(true, k_adjs_product, gr, 256, 0, st, "k_adjs_product", tr, C, p->R, p->nl_coef, P[s], Q)))
       return rc;
-    if ((rc = forward_real(p, batch * C, Q, outs[s], false, st))) return rc;
+    if ((rc = forward_real(p, batch * C, Q, outs[s], true, st))) return rc;
   }
 
   // backward
-  if ((rc = launch_pdl(false, k_adjs_begin, gh, 256, 0, st, "k_adjs_begin", T, th, C, (const float2*)ubar_next, uu, n0, n1,
+  if ((rc = launch_pdl(true, k_adjs_begin, gh, 256, 0, st, "k_adjs_begin", T, th, C, (const float2*)ubar_next, uu, n0, n1,
                        n2, n3, ubar_acc, n0b, n1b, n2b, nbs, tbar)))
     return rc;
   AdjEnd e{F, uu, a1, n0, n1, n2, ubar_acc, a1b, n0b, n1b, n2b, nbs, (float2*)ubar, tbar};
   const float scale = p->nl_coef * (float)p->R;
   for (int s = 3; s >= 0; --s) {
     // w = coef N irfft(nbar); ubar_c = sum_c' w_c' d_c u_c', u_i w_c -> rfft -> combination
-    if ((rc = inverse_real(p, batch * C, nbs, nbp, false, st))) return rc;
+    if ((rc = inverse_real(p, batch * C, nbs, nbp, true, st))) return rc;
     const float* Ps = P[s];
     const float* g1 = nd > 1 ? Ps + 2 * tr : nullptr;
     const float* g2 = nd > 2 ? Ps + 3 * tr : nullptr;
     const auto vjp = nd == 1 ? k_adj_vjp_products<1> : nd == 2 ? k_adj_vjp_products<2> : k_adj_vjp_products<3>;
-    if ((rc = launch_pdl(false, vjp, gr / C + 1, 256, 0, st, "k_adj_vjp_products", batch, p->R, scale, nbp, Ps, Ps + tr, g1,
+    if ((rc = launch_pdl(true, vjp, gr / C + 1, 256, 0, st, "k_adj_vjp_products", batch, p->R, scale, nbp, Ps, Ps + tr, g1,
                          g2, Q, Q + tr)))
       return rc;
-    if ((rc = forward_real(p, nb * batch * C, Q, F, false, st))) return rc;
-    if ((rc = launch_pdl(false, k_adjs_end, gh, 256, 0, st, "k_adjs_end", g, T, th, C, (float)(1.0 / (double)p->R), s, e)))
+    if ((rc = forward_real(p, nb * batch * C, Q, F, true, st))) return rc;
+    if ((rc = launch_pdl(true, k_adjs_end, gh, 256, 0, st, "k_adjs_end", g, T, th, C, (float)(1.0 / (double)p->R), s, e)))
       return rc;
   }
   return FSM_OK;

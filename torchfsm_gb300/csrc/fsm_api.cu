@@ -702,7 +702,6 @@ size_t integrate_workspace_bytes(const FsmPlan* p, int32_t batch, int32_t steps)
 }  // namespace fsm
 
 namespace fsm {
-bool short_grid(const FsmPlan* p, int64_t fields);
 // Batches at or above kSplitPoints spectral points run in parts of about kPartPoints points
 // (2 to kMaxParts parts, at most one per sample) on as many streams. Measured on 256^2 x 64
 // (2.1 M points): one sequence 322 us per step, 2 parts 284, 4 parts 270, 8 parts 261.
@@ -961,6 +960,7 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   a.n_frames = n_frames;
   a.slots = record_slot ? d_slots : nullptr;
   a.dc = (float2*)(ws + align256((size_t)(steps + 1) * sizeof(int32_t)));
+  a.pdl = prof == nullptr;  // the profiled call times each launch by itself
 
   if (p->path == 3) return timed(prof, kProfOther, [&] { return launch_pointwise(p, a, st); });
   if (p->path == 1) return timed(prof, kProfOther, [&] { return launch_line(p, a, st); });
@@ -988,7 +988,6 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   const int NP = (!allow_split || prof || cap != cudaStreamCaptureStatusNone) ? 1 : fsm::split_parts(p, batch);
   const bool split = NP > 1;
   if (!split) {
-    a.pdl = short_grid(p, (int64_t)batch * p->C);
     PlaneSequence q{p, batch_arrays(p, a, arr, 0, batch), record_slot, steps, st, prof};
     if ((rc = q.prime())) return rc;
     for (int k = 0; k < steps; ++k)
@@ -1044,12 +1043,6 @@ int integrate_with_workspace(const FsmPlan* p, int32_t batch, void* state, int32
 }  // namespace fsm
 
 namespace fsm {
-// Whether a pass over `fields` fields is short enough for its tail and the next one's start to
-// matter (launch_pdl): up to 2 M spectral points. 3D Burgers 64^3 x 3 (1.2 M points): 5.03 -> 4.39 ms
-// per 20 steps; 256^3 (25 M): 14.3 -> 15.2 ms per 4, so longer passes launch plainly, as do the
-// adjoint step's kernels in their captured graph (22.2 -> 23.2 ms per iteration of 128^2 x 16).
-bool short_grid(const FsmPlan* p, int64_t fields) { return fields * p->S <= ((int64_t)1 << 21); }
-
 int forward_real(const FsmPlan* p, int64_t count, const float* in, float2* out, bool pdl, cudaStream_t st) {
   if (count == 0) return FSM_OK;
   const int nd = p->ndim;
@@ -1113,12 +1106,12 @@ int fsm_integrate_profiled(const FsmPlan* p, int32_t batch, void* state, int32_t
 
 int fsm_rfftn(const FsmPlan* p, int32_t count, const float* in, void* out, void* stream) {
   if (!p || !in || !out || count < 0) return set_error(FSM_ERR_INVALID, "rfftn arguments");
-  return fsm::forward_real(p, count, in, (float2*)out, fsm::short_grid(p, count), (cudaStream_t)stream);
+  return fsm::forward_real(p, count, in, (float2*)out, true, (cudaStream_t)stream);
 }
 
 int fsm_irfftn(const FsmPlan* p, int32_t count, void* in, float* out, void* stream) {
   if (!p || !in || !out || count < 0) return set_error(FSM_ERR_INVALID, "irfftn arguments");
-  return fsm::inverse_real(p, count, (float2*)in, out, fsm::short_grid(p, count), (cudaStream_t)stream);
+  return fsm::inverse_real(p, count, (float2*)in, out, true, (cudaStream_t)stream);
 }
 
 int fsm_nonfinite_flags(const FsmPlan* p, int32_t count, const void* fields, int32_t* flags, void* stream) {

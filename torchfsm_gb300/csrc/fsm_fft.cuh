@@ -60,12 +60,18 @@ __device__ __forceinline__ float2 cfma(float2 c, float2 b, float2 a) {
   return make_float2(fmaf(c.x, b.x, fmaf(-c.y, b.y, a.x)), fmaf(c.x, b.y, fmaf(c.y, b.x, a.y)));
 }
 
-// Programmatic dependent launch (launch_pdl): let the next grid in the stream be placed, and wait for
-// the grid before this one; both do nothing in a plain launch.
-__device__ __forceinline__ void pdl_wait() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+// Programmatic dependent launch (launch_pdl): wait for the grid before this one; let the next grid in
+// the stream be placed. Both do nothing in a plain launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel's `__restrict__` pointer parameter after pdl_wait(): loads through the parameter itself may be
+// moved ahead of the wait (nothing else is taken to write that memory while the kernel runs); loads
+// through the returned pointer may not. Pointers that come in a struct need no such care.
+template <class T>
+__device__ __forceinline__ T* pdl_ptr(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
 }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <bool INV>
 __device__ __forceinline__ void dft2(float2* v) {

@@ -139,11 +139,13 @@ bool resident_config(const FsmPlan* p, int batch, ResConfig* out);
 int launch_resident(const FsmPlan* p, const ResConfig& c, const StepArgs& a, cudaStream_t st);
 
 // Programmatic dependent launch: the grid may start (its blocks are placed, constants are loaded)
-// while the one before it in the stream still runs; the kernel waits in pdl_wait() before it touches
+// while the one before it in the stream drains; the kernel waits in pdl_wait() before it touches
 // anything that grid wrote or still reads. Every kernel launched this way calls pdl_wait() in every
-// thread before its first access to global memory other than the plan's twiddles and wavenumbers.
-// For chains of short kernels (short_grid, fsm_api.cu); not used for the parts
-// of a split batch, whose waiting blocks would take the places of other parts' running ones.
+// thread before its first access to global memory other than the plan's twiddles and wavenumbers,
+// and pdl_trigger() late, before its last transform: triggered at the start, the next grids' waiting
+// blocks took the places of running ones (512^2 x 5: 6.26 ms per 40 steps, 3D Burgers 256^3 15.2 ms
+// per 4). Plain launches -> triggered late: vorticity 512^2 x 5 6.31 -> 5.33 ms, 256^2 x 64 8.61 ->
+// 8.31 ms per 50 steps, 3D Burgers 64^3 x 3 5.03 -> 4.30 ms per 20, 256^3 no change.
 template <class... P, class... A>
 inline int launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                       const char* what, A&&... args) {

@@ -23,6 +23,7 @@ __global__ void k_ks_mean(StepArgs a, int nx) {
     const int b = i / nx, x = i % nx;
     acc += a.prod[((int64_t)b * a.n_prod) * a.ms + (int64_t)x * a.wp].x;
   }
+  pdl_trigger();
   __shared__ float red[256];
   red[threadIdx.x] = acc;
   __syncthreads();

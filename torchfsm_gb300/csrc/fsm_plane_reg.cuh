@@ -480,6 +480,7 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, i
       axis0_update_any<NX, KIND, DIM>(a, st, smem + Cfg::WORDS, b, j0, t, cg, last);
     }
   }
+  pdl_trigger();
   if (!a.emit) return;  // uniform
   // 2D: columns from hk on are dealiased and the row pass does not read them: nothing to store.
   // 3D: the next passes read the columns (jm, jl) with jm kept and jl < hk.
@@ -651,6 +652,7 @@ __device__ __forceinline__ void plane_row_body(const StepArgs& a, int blk, int b
     float2 zp[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) zp[j] = make_float2(p[0][j], p[1][j]);
+    pdl_trigger();
     reg_fft<NY, false>(zp, scr, twt, t);
     split_store_r<NY>(zp, t, lane, prod + (int64_t)r0 * WP, prod + (int64_t)(r0 + 1) * WP);
   } else {
@@ -704,6 +706,7 @@ __device__ __forceinline__ void plane_row_body(const StepArgs& a, int blk, int b
         acc[j].x += u1[j] * Z2[j].x;
         acc[j].y += u1[j] * Z2[j].y;
       }
+      if (rr == 1) pdl_trigger();
       reg_fft<NY, false>(acc, scr, twt, t);
       split_store_r<NY>(acc, t, lane, prod + roff, prod + S + roff);
     }

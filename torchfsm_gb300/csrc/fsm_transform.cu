@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_r2c_last(const float* __
   float2* z = smem + N + g * N;
   load_twiddles(tw, master, kTwiddleMax, N, threadIdx.x, Cfg::THREADS);
   pdl_wait();
+  in = pdl_ptr(in);
   const int64_t r0 = ((int64_t)blockIdx.x * Cfg::GROUPS + g) * 2;
   const bool has0 = r0 < rows, has1 = r0 + 1 < rows;
   for (int n = t; n < N; n += Cfg::G) {
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_r2c_last(const float* __
     z[n] = make_float2(a, b);
   }
   __syncthreads();
+  pdl_trigger();
   fft<N, Cfg::G, Cfg::BLOCK, false>(z, tw, t);
   for (int k = t; k < H; k += Cfg::G) {
     const float2 zk = z[k];
@@ -61,6 +63,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_c2r_last(const float2* _
   float2* z = smem + N + g * N;
   load_twiddles(tw, master, kTwiddleMax, N, threadIdx.x, Cfg::THREADS);
   pdl_wait();
+  in = pdl_ptr(in);
   const int64_t r0 = ((int64_t)blockIdx.x * Cfg::GROUPS + g) * 2;
   const bool has0 = r0 < rows, has1 = r0 + 1 < rows;
   for (int k = t; k < H; k += Cfg::G) {
@@ -74,6 +77,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) k_c2r_last(const float2* _
     if (k > 0 && k < N / 2) z[N - k] = make_float2(A.x + B.y, B.x - A.y);  // conj(A) + i conj(B)
   }
   __syncthreads();
+  pdl_trigger();
   fft<N, Cfg::G, Cfg::BLOCK, true>(z, tw, t);
   for (int n = t; n < N; n += Cfg::G) {
     const float2 v = z[n];

@@ -37,9 +37,9 @@ __global__ void __launch_bounds__(256) k_c2c_strided_r(float2* __restrict__ data
   float2* scr = tile + W * P;
   const int g = threadIdx.x / T, t = threadIdx.x % T;
   const int64_t c0 = (int64_t)blockIdx.x * W;
-  float2* base = data + (int64_t)blockIdx.y * N * inner;
   load_reg_twiddles<N>(twt, master, threadIdx.x, 256);
   pdl_wait();
+  float2* base = pdl_ptr(data) + (int64_t)blockIdx.y * N * inner;
   {
     float2 buf[N * W / 256];
 #pragma unroll
@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(256) k_c2c_strided_r(float2* __restrict__ data
   float2 v[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) v[j] = tile[g * P + t + T * j];
+  pdl_trigger();
   reg_fft<N, INV>(v, scr + g * P, twt, t);
 #pragma unroll
   for (int j = 0; j < E; ++j) tile[g * P + t + T * j] = v[j];
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(256) k_axis1_inv_r(StepArgs a) {
     reg_fft<NY, true>(v, tC + g * P, twt, t);
 #pragma unroll
     for (int j = 0; j < E; ++j) tC[g * P + t + T * j] = v[j];
+    pdl_trigger();
     reg_fft<NY, true>(w, tA + g * P, twt, t);
 #pragma unroll
     for (int j = 0; j < E; ++j) tA[g * P + t + T * j] = w[j];
@@ -314,6 +316,7 @@ __global__ void __launch_bounds__(256, 2) k_axis2_r(StepArgs a) {
       split_one<NZ>(Z, t, lane, prod + roff, prod + S + roff);
 #pragma unroll
       for (int j = 0; j < E; ++j) Z[j] = make_float2(c2v[j], 0.f);
+      if (rr == 1) pdl_trigger();
       reg_fft<NZ, false>(Z, scr, twt, t);
       split_one<NZ>(Z, t, lane, prod + 2 * S + roff, nullptr);
     } else {
@@ -327,6 +330,7 @@ __global__ void __launch_bounds__(256, 2) k_axis2_r(StepArgs a) {
       reg_fft<NZ, true>(Z, scr, twt, t);
 #pragma unroll
       for (int j = 0; j < E; ++j) Z[j] = make_float2(p[j] + 0.5f * Z[j].x * Z[j].x, 0.f);
+      if (rr == 1) pdl_trigger();
       reg_fft<NZ, false>(Z, scr, twt, t);
       split_one<NZ>(Z, t, lane, prod + roff, nullptr);
     }
