@@ -30,3 +30,17 @@ def test_rates_on_unequal_axes(rate, term, shape):
     got = op.integrate(u_0=torch.tensor(u0, device="cuda"), mesh=mesh, dt=2e-3, step=4)
     ref, _ = S.integrate(u0.astype("float64"), mesh, lin, nl, 2e-3, 4, de_aliasing_rate=rate)
     assert S.rel_l2(got.cpu().numpy(), ref) < 1e-5  # the parity tests' bound
+
+
+# the plane kernel at the largest plane of each y length, and the first sizes beyond it
+@pytest.mark.parametrize("shape", [(16, 16, 256), (16, 32, 128), (16, 64, 64), (16, 128, 32), (16, 256, 16), (16, 64, 128),
+                                   (16, 32, 32)])
+@pytest.mark.parametrize("term", ["convection", "leray"])
+def test_plane_kernel_sizes(term, shape):
+    op = pde.Burgers(0.05) if term == "convection" else pde.NavierStokes(20)
+    nl = [(-1.0, "convection")] if term == "convection" else [(1.0, "ns_pressure_convection")]
+    mesh = [(0, 2 * math.pi, n) for n in shape]
+    u0 = initial.band_limited(shape, 2, 3, 3, 6, 0.3).astype("float32")
+    got = op.integrate(u_0=torch.tensor(u0, device="cuda"), mesh=mesh, dt=1e-3, step=3)
+    ref, _ = S.integrate(u0.astype("float64"), mesh, [(0.05, ("laplacian",))], nl, 1e-3, 3)
+    assert S.rel_l2(got.cpu().numpy(), ref) < 1e-5  # the parity tests' bound

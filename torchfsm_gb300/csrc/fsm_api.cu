@@ -631,7 +631,7 @@ int fsm_plan_launch_count(const FsmPlan* plan, int32_t batch, int32_t steps, int
   if (fsm::resident_config(plan, batch, &res)) {
     *launches = steps > 0 ? (steps + kResidentSteps - 1) / kResidentSteps : 1;
   } else if (plan->path == 2 || plan->path == 4) {
-    const int64_t per_stage = (plan->path == 4 ? 4 : 2) +
+    const int64_t per_stage = (plan->path == 4 && !fsm::volume_plane_applies(plan) ? 4 : 2) +
                               ((plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) ? 1 : 0);
     *launches = (int64_t)fsm::split_parts(plan, batch) * (1 + (int64_t)steps * plan->nstages * per_stage);
   } else if (plan->path == 1 && plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) {
@@ -845,7 +845,9 @@ struct PlaneSequence {
     const bool ks_mean = p->nl == FSM_NL_KS && (p->flags & FSM_FLAG_REMOVE_MEAN);
     const bool vol = p->path == 4;
     for (int s = 0; s < p->nstages; ++s) {
-      if (vol) {
+      if (vol && volume_plane_applies(p)) {
+        if ((rc = timed(prof, kProfRow, [&] { return launch_volume_plane(p, a, st); }))) return rc;
+      } else if (vol) {
         if ((rc = timed(prof, kProfOther, [&] { return launch_volume_axis1_inv(p, a, st); }))) return rc;
         if ((rc = timed(prof, kProfRow, [&] { return launch_volume_axis2(p, a, st); }))) return rc;
         if ((rc = timed(prof, kProfOther, [&] { return launch_volume_axis1_fwd(p, a, st); }))) return rc;

@@ -81,6 +81,9 @@ int integrate_on_workspace(const FsmPlan* p, int32_t batch, void* state, int32_t
 // Recompute the coefficient tables of batch entries [b0, b0 + n) for time step dt (one launch).
 int set_batch_dt_range(FsmPlan* p, int32_t b0, int32_t n, double dt, cudaStream_t st);
 
+// The three passes between the x passes in one launch where planes are small (fsm_volume_plane.cu).
+bool volume_plane_applies(const FsmPlan* p);
+int launch_volume_plane(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_volume_axis1_inv(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_volume_axis2(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_volume_axis1_fwd(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
