@@ -179,3 +179,38 @@ def test_table_derivatives_of_the_library_match_the_contour_formulas():
         # at |z| = 0.5 the closed forms lose 4/z^4 x 2^-53 x ~10 = 7e-14 of values of order 0.1
         scale = ref[t].abs().max()
         assert float((out[t] - ref[t]).abs().max() / scale) < 1e-11, t
+
+
+@pytest.mark.parametrize("shape,batch", [((16, 16), 1), ((32, 64), 3), ((64, 32), 2), ((16, 128), 5), ((128, 256), 1),
+                                         ((16, 512), 2), ((512, 16), 1)])
+def test_2d_step_adjoint_every_row_length(shape, batch):
+    """The fused row kernel of the 2D adjoint step at every last-axis length, batches of one and odd
+    ones, against the step written as FP32 tensor arithmetic."""
+    from torchfsm_gb300 import adjoint, initial
+
+    dev = torch.device("cuda", 0)
+    dt = 1e-3
+    mesh = [(0.0, 2 * np.pi, n) for n in shape]
+    op = 0.02 * Laplacian() - Convection()
+    u0 = torch.tensor(initial.band_limited(shape, batch, 2, 5, 3, 0.5), dtype=torch.float32, device=dev)
+    with torch.no_grad():
+        op.integrate(u_0=u0, mesh=mesh, dt=dt, step=1)
+    plan = op._state_dict["integrator"].plan
+    h = shape[-1] // 2 + 1
+    L64 = op._linear_coef64(dev)
+    L64 = L64.expand(L64.shape[:2] + tuple(shape))[..., :h]
+    adj = adjoint.ConvectionAdjoint(plan, plan.program, L64, dt)
+    u = adj.sp.to_half(u0).contiguous()
+    ub = (adj.sp.to_half(torch.tensor(initial.band_limited(shape, batch, 2, 7, 4, 1.0), dtype=torch.float32,
+                                      device=dev)) / adj.ntot).contiguous()
+    tb = torch.zeros((6,) + tuple(u.shape), dtype=torch.float64, device=dev)
+    tb_ref = torch.zeros_like(tb)
+    out, ref = adj.step_adjoint(u, ub, tb), _torch_step_adjoint(adj, u, ub, tb_ref)
+    torch.cuda.synchronize()
+
+    def rel(a, b):
+        return float((a - b).abs().pow(2).sum().sqrt() / b.abs().pow(2).sum().sqrt())
+
+    assert rel(out, ref) <= 1e-5  # the bound of the same comparison above
+    for t in range(6):
+        assert rel(tb[t], tb_ref[t]) <= 1e-5, t

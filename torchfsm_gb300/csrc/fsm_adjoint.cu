@@ -427,6 +427,8 @@ int fsm_step_adjoint(const FsmPlan* p, int32_t batch, const void* u, const void*
   AdjTabs T{p->tab, p->tstride, p->lin_batch, p->lin_ch, p->S};
   const unsigned gh = grid_for(th), gr = grid_for(tr);
 
+  const float inv_n = (float)(1.0 / (double)p->R);
+
   // forward stages, keeping each stage's physical fields for its vector-Jacobian product
   const float2* xs[4] = {uu, uu, uu, a1};
   const float2* ys[4] = {nullptr, n0, n1, n2};
@@ -437,6 +439,13 @@ int fsm_step_adjoint(const FsmPlan* p, int32_t batch, const void* u, const void*
     if ((rc = launch_pdl(true, k_adjs_fields, gh, 256, 0, st, "k_adjs_fields", g, T, th, C, (int)(s > 0), xs[s], ys[s],
                          al[s], zs[s], be[s], s == 1 ? a1 : nullptr, F)))
       return rc;
+    if (nd == 2) {
+      if ((rc = transform_c2c_strided(p->n[0], true, F, nb * batch * C, p->h, p->tw, true, st))) return rc;
+      if ((rc = launch_adj_row(p->n[1], AdjRow{F, P[s], outs[s], p->tw, th, tr, inv_n, p->nl_coef, batch, p->n[0], 0}, st)))
+        return rc;
+      if ((rc = transform_c2c_strided(p->n[0], false, outs[s], batch * C, p->h, p->tw, true, st))) return rc;
+      continue;
+    }
     if ((rc = inverse_real(p, nb * batch * C, F, P[s], true, st))) return rc;
     if ((rc = launch_pdl(true, k_adjs_product, gr, 256, 0, st, "k_adjs_product", tr, C, p->R, p->nl_coef, P[s], Q)))
       return rc;
@@ -451,16 +460,23 @@ int fsm_step_adjoint(const FsmPlan* p, int32_t batch, const void* u, const void*
   const float scale = p->nl_coef * (float)p->R;
   for (int s = 3; s >= 0; --s) {
     // w = coef N irfft(nbar); ubar_c = sum_c' w_c' d_c u_c', u_i w_c -> rfft -> combination
-    if ((rc = inverse_real(p, batch * C, nbs, nbp, true, st))) return rc;
-    const float* Ps = P[s];
-    const float* g1 = nd > 1 ? Ps + 2 * tr : nullptr;
-    const float* g2 = nd > 2 ? Ps + 3 * tr : nullptr;
-    const auto vjp = nd == 1 ? k_adj_vjp_products<1> : nd == 2 ? k_adj_vjp_products<2> : k_adj_vjp_products<3>;
-    if ((rc = launch_pdl(true, vjp, gr / C + 1, 256, 0, st, "k_adj_vjp_products", batch, p->R, scale, nbp, Ps, Ps + tr, g1,
-                         g2, Q, Q + tr)))
-      return rc;
-    if ((rc = forward_real(p, nb * batch * C, Q, F, true, st))) return rc;
-    if ((rc = launch_pdl(true, k_adjs_end, gh, 256, 0, st, "k_adjs_end", g, T, th, C, (float)(1.0 / (double)p->R), s, e)))
+    if (nd == 2) {
+      if ((rc = transform_c2c_strided(p->n[0], true, nbs, batch * C, p->h, p->tw, true, st))) return rc;
+      if ((rc = launch_adj_row(p->n[1], AdjRow{nbs, P[s], F, p->tw, th, tr, inv_n, scale, batch, p->n[0], 1}, st)))
+        return rc;
+      if ((rc = transform_c2c_strided(p->n[0], false, F, nb * batch * C, p->h, p->tw, true, st))) return rc;
+    } else {
+      if ((rc = inverse_real(p, batch * C, nbs, nbp, true, st))) return rc;
+      const float* Ps = P[s];
+      const float* g1 = nd > 1 ? Ps + 2 * tr : nullptr;
+      const float* g2 = nd > 2 ? Ps + 3 * tr : nullptr;
+      const auto vjp = nd == 1 ? k_adj_vjp_products<1> : k_adj_vjp_products<3>;
+      if ((rc = launch_pdl(true, vjp, gr / C + 1, 256, 0, st, "k_adj_vjp_products", batch, p->R, scale, nbp, Ps, Ps + tr, g1,
+                           g2, Q, Q + tr)))
+        return rc;
+      if ((rc = forward_real(p, nb * batch * C, Q, F, true, st))) return rc;
+    }
+    if ((rc = launch_pdl(true, k_adjs_end, gh, 256, 0, st, "k_adjs_end", g, T, th, C, inv_n, s, e)))
       return rc;
   }
   return FSM_OK;

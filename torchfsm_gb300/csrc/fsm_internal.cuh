@@ -90,6 +90,21 @@ int launch_volume_axis1_fwd(const FsmPlan* p, const StepArgs& a, cudaStream_t st
 
 int launch_line(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 
+// The row kernel of a 2D adjoint step (fsm_adjoint_row.cu): B samples of two channels, n0 rows; half-spectrum
+// arrays [..][B][2][n0][H] (th values a field pair), physical ones [..][B][2][n0][NY] (tr values).
+// Forward: in[3] -> P[3] and out. Backward: in, P[3] -> out[3]. inv: 1 / points; scale: the coefficient
+// (backward: times the points).
+struct AdjRow {
+  const float2* in;
+  float* P;
+  float2* out;
+  const float2* tw;
+  int64_t th, tr;
+  float inv, scale;
+  int B, n0, backward;
+};
+int launch_adj_row(int ny, const AdjRow& a, cudaStream_t st);
+
 // One launch of the 1D line kernel over the samples of several plans of different lengths
 // (256..4096 points, one nonlinear kind): entry j advances a[j].B samples of a[j] by a[j].steps
 // steps (the same for every entry), without recording. cta0 is filled in by the launcher.
