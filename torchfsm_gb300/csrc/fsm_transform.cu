@@ -5,106 +5,203 @@
 // mesh.py:481-491) for the initial spectrum, the returned fields and the
 // recorded trajectories.
 #include "fsm_internal.cuh"
+#include "fsm_linefft.cuh"
 
 namespace fsm {
 
-template <int N>
-struct RowCfg {
-  static constexpr int G = (N / 16 < 32) ? 32 : N / 16;
-  static constexpr bool BLOCK = G > 32;
-  static constexpr int GROUPS = BLOCK ? 1 : 8;
-  static constexpr int THREADS = G * GROUPS;
-  static constexpr size_t SMEM = (size_t)(GROUPS + 1) * N * sizeof(float2);
-};
+// Rows of up to 512 points: a group of T lanes per pair of rows, registers from the loads to the
+// stores (lanes on adjacent elements). Longer rows: T threads per pair (fsm_linefft.cuh). Bound: launch
+// latency for few rows, else memory. The shared-memory Stockham passes these replaced, us per launch of
+// 256^2 x 16 / 1024 x 7 / 4096 x 32: r2c 10.0 / 19.8 / 21.2, c2r 7.9 / 15.8 / 17.0; now
+// 5.4 / 7.4 / 12.0 and 5.2 / 7.5 / 11.9.
 
 // rows: [rows][N] real -> [rows][N/2+1] complex (unnormalised forward)
 template <int N>
-__global__ void __launch_bounds__(RowCfg<N>::THREADS) k_r2c_last(const float* __restrict__ in, float2* __restrict__ out,
-                                                                  int64_t rows, const float2* __restrict__ master) {
-  using Cfg = RowCfg<N>;
-  constexpr int H = N / 2 + 1;
+__global__ void __launch_bounds__(256) k_r2c_last(const float* __restrict__ in, float2* __restrict__ out, int64_t rows,
+                                                  const float2* __restrict__ master) {
+  constexpr int T = RegShape<N>::T, E = RegShape<N>::E, H = N / 2 + 1, J = N / (2 * T);
   extern __shared__ float2 smem[];
-  float2* tw = smem;
-  const int g = threadIdx.x / Cfg::G;
-  const int t = threadIdx.x % Cfg::G;
-  float2* z = smem + N + g * N;
-  load_twiddles(tw, master, kTwiddleMax, N, threadIdx.x, Cfg::THREADS);
+  const int lane = threadIdx.x & 31, g = threadIdx.x / T, t = threadIdx.x % T;
+  load_reg_twiddles<N>(smem, master, threadIdx.x, blockDim.x);
   pdl_wait();
   in = pdl_ptr(in);
-  const int64_t r0 = ((int64_t)blockIdx.x * Cfg::GROUPS + g) * 2;
-  const bool has0 = r0 < rows, has1 = r0 + 1 < rows;
-  for (int n = t; n < N; n += Cfg::G) {
-    const float a = has0 ? in[r0 * N + n] : 0.f;
-    const float b = has1 ? in[(r0 + 1) * N + n] : 0.f;
-    z[n] = make_float2(a, b);
-  }
   __syncthreads();
-  pdl_trigger();
-  fft<N, Cfg::G, Cfg::BLOCK, false>(z, tw, t);
-  for (int k = t; k < H; k += Cfg::G) {
-    const float2 zk = z[k];
-    const float2 zm = cconj(z[(N - k) & (N - 1)]);
-    if (has0) out[r0 * H + k] = cscale(cadd(zk, zm), 0.5f);
-    if (has1) out[(r0 + 1) * H + k] = cscale(cmulmi(csub(zk, zm)), 0.5f);
+  const int64_t r0 = ((int64_t)blockIdx.x * (blockDim.x / T) + g) * 2;
+  const bool has0 = r0 < rows, has1 = r0 + 1 < rows;
+  float2 v[E];
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    const int n = t + T * j;
+    v[j] = make_float2(has0 ? in[r0 * N + n] : 0.f, has1 ? in[(r0 + 1) * N + n] : 0.f);
   }
+  pdl_trigger();
+  reg_fft<N, false>(v, smem + N + g * reg_scratch<N>(), smem, t);
+  const int partner_lane = (lane & ~(T - 1)) | ((T - t) & (T - 1));
+#pragma unroll
+  for (int j = 0; j <= J; ++j) {
+    const float2 send = v[E - 1 - j];
+    float2 recv;
+    recv.x = __shfl_sync(0xffffffffu, send.x, partner_lane);
+    recv.y = __shfl_sync(0xffffffffu, send.y, partner_lane);
+    const float2 zm = cconj((t == 0) ? v[(E - j) & (E - 1)] : recv);
+    const int k = t + T * j;
+    if (k <= N / 2) {
+      if (has0) out[r0 * H + k] = cscale(cadd(v[j], zm), 0.5f);
+      if (has1) out[(r0 + 1) * H + k] = cscale(cmulmi(csub(v[j], zm)), 0.5f);
+    }
+  }
+}
+
+// A + i B at index k of the Hermitian extensions of two half rows.
+template <int N>
+__device__ __forceinline__ float2 herm_value(const float2* a, const float2* b, int k) {
+  const bool hi = k > N / 2;
+  const int kk = hi ? N - k : k;
+  float2 A = a ? a[kk] : make_float2(0.f, 0.f), B = b ? b[kk] : make_float2(0.f, 0.f);
+  if (kk == 0 || kk == N / 2) A.y = B.y = 0.f;
+  if (hi) {
+    A.y = -A.y;
+    B.y = -B.y;
+  }
+  return make_float2(A.x - B.y, A.y + B.x);
 }
 
 // rows: [rows][N/2+1] complex -> [rows][N] real, times `scale`
 template <int N>
-__global__ void __launch_bounds__(RowCfg<N>::THREADS) k_c2r_last(const float2* __restrict__ in, float* __restrict__ out,
-                                                                  int64_t rows, float scale,
-                                                                  const float2* __restrict__ master) {
-  using Cfg = RowCfg<N>;
-  constexpr int H = N / 2 + 1;
+__global__ void __launch_bounds__(256) k_c2r_last(const float2* __restrict__ in, float* __restrict__ out, int64_t rows,
+                                                  float scale, const float2* __restrict__ master) {
+  constexpr int T = RegShape<N>::T, E = RegShape<N>::E, H = N / 2 + 1;
   extern __shared__ float2 smem[];
-  float2* tw = smem;
-  const int g = threadIdx.x / Cfg::G;
-  const int t = threadIdx.x % Cfg::G;
-  float2* z = smem + N + g * N;
-  load_twiddles(tw, master, kTwiddleMax, N, threadIdx.x, Cfg::THREADS);
+  const int g = threadIdx.x / T, t = threadIdx.x % T;
+  load_reg_twiddles<N>(smem, master, threadIdx.x, blockDim.x);
   pdl_wait();
   in = pdl_ptr(in);
-  const int64_t r0 = ((int64_t)blockIdx.x * Cfg::GROUPS + g) * 2;
-  const bool has0 = r0 < rows, has1 = r0 + 1 < rows;
-  for (int k = t; k < H; k += Cfg::G) {
-    float2 A = has0 ? in[r0 * H + k] : make_float2(0.f, 0.f);
-    float2 B = has1 ? in[(r0 + 1) * H + k] : make_float2(0.f, 0.f);
-    if (k == 0 || k == N / 2) {
-      A.y = 0.f;
-      B.y = 0.f;
-    }
-    z[k] = make_float2(A.x - B.y, A.y + B.x);  // A + i B
-    if (k > 0 && k < N / 2) z[N - k] = make_float2(A.x + B.y, B.x - A.y);  // conj(A) + i conj(B)
-  }
   __syncthreads();
+  const int64_t r0 = ((int64_t)blockIdx.x * (blockDim.x / T) + g) * 2;
+  const float2* a = r0 < rows ? in + r0 * H : nullptr;
+  const float2* b = r0 + 1 < rows ? in + (r0 + 1) * H : nullptr;
+  float2 v[E];
+#pragma unroll
+  for (int j = 0; j < E; ++j) v[j] = herm_value<N>(a, b, t + T * j);
   pdl_trigger();
-  fft<N, Cfg::G, Cfg::BLOCK, true>(z, tw, t);
-  for (int n = t; n < N; n += Cfg::G) {
-    const float2 v = z[n];
-    if (has0) out[r0 * N + n] = v.x * scale;
-    if (has1) out[(r0 + 1) * N + n] = v.y * scale;
+  reg_fft<N, true>(v, smem + N + g * reg_scratch<N>(), smem, t);
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    const int n = t + T * j;
+    if (a) out[r0 * N + n] = v[j].x * scale;
+    if (b) out[(r0 + 1) * N + n] = v[j].y * scale;
   }
+}
+
+template <int N>
+__global__ void __launch_bounds__(LineCfg<N>::T) k_r2c_line(const float* __restrict__ in, float2* __restrict__ out,
+                                                            int64_t rows, const float2* __restrict__ master) {
+  using Cfg = LineCfg<N>;
+  constexpr int T = Cfg::T, E = Cfg::E, H = Cfg::H;
+  extern __shared__ float2 smem[];
+  float2 *buf0 = smem + Cfg::TW, *buf1 = buf0 + Cfg::NB;
+  const int t = threadIdx.x;
+  line_twiddles<N>(smem, master, t, T);
+  pdl_wait();
+  in = pdl_ptr(in);
+  __syncthreads();
+  const int64_t r0 = (int64_t)blockIdx.x * 2;
+  const bool has1 = r0 + 1 < rows;
+  float2 v[E];
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    const int n = t + T * j;
+    v[j] = make_float2(in[r0 * N + n], has1 ? in[(r0 + 1) * N + n] : 0.f);
+  }
+  pdl_trigger();
+  line_passes<N, false, 1>(v, buf0, buf1, smem, t, 0, true);
+  // Z(N - k) of the upper half through the buffer that the next exchange would take
+  float2* x = (line_exchanges<N>() & 1) ? buf1 : buf0;
+#pragma unroll
+  for (int j = E / 2; j < E; ++j) x[line_pad(t + T * j)] = v[j];
+  if (t == 0) x[0] = v[0];
+  line_sync<N>(0);
+#pragma unroll
+  for (int j = 0; j <= E / 2; ++j) {
+    const int k = t + T * j;
+    if (k > N / 2) break;
+    const float2 zm = cconj(x[line_pad((N - k) & (N - 1))]);
+    out[r0 * H + k] = cscale(cadd(v[j], zm), 0.5f);
+    if (has1) out[(r0 + 1) * H + k] = cscale(cmulmi(csub(v[j], zm)), 0.5f);
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__(LineCfg<N>::T) k_c2r_line(const float2* __restrict__ in, float* __restrict__ out,
+                                                            int64_t rows, float scale,
+                                                            const float2* __restrict__ master) {
+  using Cfg = LineCfg<N>;
+  constexpr int T = Cfg::T, E = Cfg::E, H = Cfg::H;
+  extern __shared__ float2 smem[];
+  float2 *buf0 = smem + Cfg::TW, *buf1 = buf0 + Cfg::NB;
+  const int t = threadIdx.x;
+  line_twiddles<N>(smem, master, t, T);
+  pdl_wait();
+  in = pdl_ptr(in);
+  __syncthreads();
+  const int64_t r0 = (int64_t)blockIdx.x * 2;
+  const float2* a = in + r0 * H;
+  const float2* b = r0 + 1 < rows ? a + H : nullptr;
+  float2 v[E];
+#pragma unroll
+  for (int j = 0; j < E; ++j) v[j] = herm_value<N>(a, b, t + T * j);
+  pdl_trigger();
+  line_passes<N, true, 1>(v, buf0, buf1, smem, t, 0, true);
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    const int n = t + T * j;
+    out[r0 * N + n] = v[j].x * scale;
+    if (b) out[(r0 + 1) * N + n] = v[j].y * scale;
+  }
+}
+
+// Threads of a launch over `pairs` row pairs of N points: whole warps, 256 at most.
+template <int N>
+static int row_threads(int64_t pairs) {
+  const int64_t need = pairs * RegShape<N>::T;
+  return need >= 256 ? 256 : (int)((need + 31) / 32 * 32);
 }
 
 template <int N>
 static int launch_r2c(const float* in, float2* out, int64_t rows, const float2* tw, bool pdl, cudaStream_t st) {
-  using Cfg = RowCfg<N>;
-  int rc = prep_smem(k_r2c_last<N>, Cfg::SMEM);
-  if (rc) return rc;
   const int64_t pairs = (rows + 1) / 2;
-  const int64_t blocks = (pairs + Cfg::GROUPS - 1) / Cfg::GROUPS;
-  return launch_pdl(pdl, k_r2c_last<N>, (unsigned)blocks, Cfg::THREADS, Cfg::SMEM, st, "k_r2c_last", in, out, rows, tw);
+  if constexpr (N <= 512) {
+    const int threads = row_threads<N>(pairs), groups = threads / RegShape<N>::T;
+    const size_t smem = (size_t)(N + groups * reg_scratch<N>()) * sizeof(float2);
+    int rc = prep_smem(k_r2c_last<N>, smem);
+    if (rc) return rc;
+    return launch_pdl(pdl, k_r2c_last<N>, (unsigned)((pairs + groups - 1) / groups), threads, smem, st, "k_r2c_last", in,
+                      out, rows, tw);
+  } else {
+    const size_t smem = (size_t)(LineCfg<N>::TW + 2 * LineCfg<N>::NB) * sizeof(float2);
+    int rc = prep_smem(k_r2c_line<N>, smem);
+    if (rc) return rc;
+    return launch_pdl(pdl, k_r2c_line<N>, (unsigned)pairs, LineCfg<N>::T, smem, st, "k_r2c_line", in, out, rows, tw);
+  }
 }
 
 template <int N>
 static int launch_c2r(const float2* in, float* out, int64_t rows, float scale, const float2* tw, bool pdl, cudaStream_t st) {
-  using Cfg = RowCfg<N>;
-  int rc = prep_smem(k_c2r_last<N>, Cfg::SMEM);
-  if (rc) return rc;
   const int64_t pairs = (rows + 1) / 2;
-  const int64_t blocks = (pairs + Cfg::GROUPS - 1) / Cfg::GROUPS;
-  return launch_pdl(pdl, k_c2r_last<N>, (unsigned)blocks, Cfg::THREADS, Cfg::SMEM, st, "k_c2r_last", in, out, rows,
-                    scale, tw);
+  if constexpr (N <= 512) {
+    const int threads = row_threads<N>(pairs), groups = threads / RegShape<N>::T;
+    const size_t smem = (size_t)(N + groups * reg_scratch<N>()) * sizeof(float2);
+    int rc = prep_smem(k_c2r_last<N>, smem);
+    if (rc) return rc;
+    return launch_pdl(pdl, k_c2r_last<N>, (unsigned)((pairs + groups - 1) / groups), threads, smem, st, "k_c2r_last", in,
+                      out, rows, scale, tw);
+  } else {
+    const size_t smem = (size_t)(LineCfg<N>::TW + 2 * LineCfg<N>::NB) * sizeof(float2);
+    int rc = prep_smem(k_c2r_line<N>, smem);
+    if (rc) return rc;
+    return launch_pdl(pdl, k_c2r_line<N>, (unsigned)pairs, LineCfg<N>::T, smem, st, "k_c2r_line", in, out, rows, scale,
+                      tw);
+  }
 }
 
 int transform_r2c_last(int n, const float* in, float2* out, int64_t rows, const float2* tw, bool pdl, cudaStream_t st) {
