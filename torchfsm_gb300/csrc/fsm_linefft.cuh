@@ -3,6 +3,7 @@
 // turn. Used by the 1D line kernel and by the last-axis transforms above 512 points.
 #pragma once
 
+#include "fsm_internal.cuh"
 #include "fsm_regfft.cuh"
 
 namespace fsm {
