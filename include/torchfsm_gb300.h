@@ -154,8 +154,9 @@ int fsm_plan_destroy(FsmPlan* plan);
 int fsm_plan_workspace_bytes(const FsmPlan* plan, int32_t batch, int32_t steps, size_t* bytes);
 
 /* Number of kernel launches fsm_integrate makes for `batch` samples and `steps` steps outside
- * stream capture (large batches run in parts, each with its own launches); batch 0 counts
- * one launch sequence (what a captured call makes). */
+ * stream capture (large batches run in parts, each with its own launches; 2D SETDRK4 solves
+ * on the resident kernel make one launch per 2048 steps); batch 0 counts one launch sequence
+ * of passes. */
 int fsm_plan_launch_count(const FsmPlan* plan, int32_t batch, int32_t steps, int64_t* launches);
 
 /* Advance `state` (half spectra, [batch][C][S] complex64, in place) by `steps`

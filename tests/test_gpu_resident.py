@@ -104,6 +104,28 @@ def test_resident_long_run_of_several_launches():
     assert torch.equal(torch.view_as_real(a), torch.view_as_real(b))
 
 
+@pytest.mark.parametrize("build,channels", [(VORT, 1), (BURG, 2)], ids=["vorticity", "convection"])
+def test_resident_captured_and_without_steps(build, channels):
+    """A captured call replays on the data it then finds; no steps leave the state as it was, recorded as frame 0."""
+    plan, sp, u, _ = _setup(build, (64, 32), 3, channels, 2e-3)
+    st0 = sp.to_half(u).contiguous()
+    ref = st0.clone()
+    plan.integrate_half(ref, 4)
+    static = torch.zeros_like(st0)
+    ws = torch.empty(plan.workspace_bytes(3, 4), dtype=torch.uint8, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.integrate_half(static, 4, workspace=ws)
+    for _ in range(2):
+        static.copy_(st0)
+        graph.replay()
+        assert torch.equal(static, ref)
+    still = st0.clone()
+    traj = torch.zeros((3, 1) + tuple(st0.shape[1:]), dtype=torch.complex64, device="cuda")
+    plan.integrate_half(still, 0, slots=[0], traj=traj)
+    assert torch.equal(still, st0) and torch.equal(traj[:, 0], st0)
+
+
 def test_resident_matches_the_fp64_oracle():
     shape, steps, dt = (64, 32), 20, 5e-3
     plan, sp, u, u0 = _setup(NSVEL, shape, 3, 2, dt)

@@ -29,7 +29,7 @@ in FP64).
 One adjoint step is one call of the library's fsm_step_adjoint (the four
 stages recomputed with the plan's own tables and the library's transforms,
 the four vector-Jacobian products above, the backward recurrence and the
-table cotangents, about 50 launches); it is captured as a CUDA graph and
+table cotangents, a few dozen launches (33 in 2D)); it is captured as a CUDA graph and
 replayed for every step. ``nonlinear`` / ``nonlinear_vjp`` state the same
 operations with tensor arithmetic for checking.
 """
@@ -251,7 +251,7 @@ class ConvectionAdjoint:
 class _StepGraph:
     """One adjoint step (``ConvectionAdjoint.step_adjoint``: recomputed stages, vector-Jacobian
     products, coefficient accumulation into ``tbar``) captured once as a CUDA graph and replayed
-    for every step; the step is a few hundred small launches, so the replay removes their host cost.
+    for every step; the step is a few dozen small launches, so the replay removes their host cost.
     Inputs are copied into the graph's static buffers; the returned cotangent is the graph's
     static output, valid until the next call."""
 

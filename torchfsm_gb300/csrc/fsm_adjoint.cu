@@ -1,7 +1,7 @@
 // The hand-written SETDRK4 adjoint (gradients of integrate, torchfsm_gb300/adjoint.py):
 // fsm_step_adjoint runs one whole adjoint step of a Convection program (the four stages
 // recomputed with the library's transforms, their vector-Jacobian products, the backward
-// recurrence and the coefficient-table cotangents) in about 50 launches; the elementwise kernels
+// recurrence and the coefficient-table cotangents) in a few dozen launches (33 in 2D); the elementwise kernels
 // of its vector-Jacobian product are also exported on their own.
 #include "fsm_internal.cuh"
 
