@@ -25,7 +25,7 @@ struct ColCfg {
 // the exchange's accesses to shared memory; the price is a CTA barrier per exchange, one each with
 // two buffers in turn (par selects the next).
 template <int NX, bool INV>
-__device__ __forceinline__ void col_fft(float2 (&v)[RegShape<NX>::E], float2* __restrict__ buf, int& par,
+__device__ __forceinline__ void col_fft(float2 (&v)[RegShape<NX>::E], float2* buf, int& par,
                                         const float2* __restrict__ twt, int t, int g) {
   using Cfg = ColCfg<NX>;
   constexpr int T = Cfg::T, E = Cfg::E, W = Cfg::W;

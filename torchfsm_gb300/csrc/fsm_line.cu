@@ -49,7 +49,7 @@ __device__ __forceinline__ float2 line_build(int k, float2 a, float mask, float 
 // a valid sample without writing global memory (spare sub-groups of a k_line_multi CTA).
 template <int N, int KIND, bool REGS>
 __device__ __forceinline__ void line_body(const StepArgs& a, int b, int t, int id, const float2* __restrict__ tw,
-                                          float2* __restrict__ reg, bool lane_on, bool active) {
+                                          float2* reg, bool lane_on, bool active) {
   using Cfg = LineCfg<N>;
   // with everything in registers the lanes beyond T repeat the work of lane t % T (same values to the
   // same shared words) instead of branching around it; they write nothing global

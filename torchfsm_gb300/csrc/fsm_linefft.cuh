@@ -61,8 +61,8 @@ __device__ __forceinline__ void line_sync(int id) {
 
 // The passes of a transform from span P on; v holds the pass's inputs (butterfly b in v[b R ..]).
 template <int N, bool INV, int P>
-__device__ __forceinline__ void line_passes(float2 (&v)[LineCfg<N>::E], float2* __restrict__ cur,
-                                            float2* __restrict__ nxt, const float2* __restrict__ tw, int t, int id,
+__device__ __forceinline__ void line_passes(float2 (&v)[LineCfg<N>::E], float2* cur,
+                                            float2* nxt, const float2* __restrict__ tw, int t, int id,
                                             bool on) {
   using Cfg = LineCfg<N>;
   constexpr int E = Cfg::E, T = Cfg::T, R = Cfg::radix(P), PER = E / R;

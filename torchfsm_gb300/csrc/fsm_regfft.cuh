@@ -117,7 +117,7 @@ constexpr int reg_scratch() {
 }
 
 template <bool INV>
-__device__ __forceinline__ void reg_fft512(float2 (&v)[16], float2* __restrict__ x, const float2* __restrict__ twt,
+__device__ __forceinline__ void reg_fft512(float2 (&v)[16], float2* x, const float2* __restrict__ twt,
                                            int t) {
   auto pad = [](int i) { return i + (i >> 4); };
   auto tw = [&](float2 a, float2 w) {
@@ -155,9 +155,11 @@ __device__ __forceinline__ void reg_fft512(float2 (&v)[16], float2* __restrict__
 
 // In-register FFT of the group's N points (see file comment). `scratch` holds
 // reg_scratch<N>() float2 private to the group; t is the lane's index in the group.
-// Every lane of the warp must call this together (warp-synchronous).
+// Every lane of the warp must call this together (warp-synchronous). The pointers to shared memory that
+// lanes exchange through (here and in the other transforms) are not __restrict__: other lanes write it, and
+// with that promise a compiler may move a lane's accesses over the barriers between.
 template <int N, bool INV>
-__device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::E], float2* __restrict__ scratch,
+__device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::E], float2* scratch,
                                         const float2* __restrict__ twt, int t) {
   if constexpr (N == 512) {
     reg_fft512<INV>(v, scratch, twt, t);
