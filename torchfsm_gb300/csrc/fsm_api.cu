@@ -633,7 +633,7 @@ int fsm_plan_launch_count(const FsmPlan* plan, int32_t batch, int32_t steps, int
   } else if (plan->path == 2 || plan->path == 4) {
     const int64_t per_stage = (plan->path == 4 && !fsm::volume_plane_applies(plan) ? 4 : 2) +
                               ((plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) ? 1 : 0);
-    *launches = (int64_t)fsm::split_parts(plan, batch) * (1 + (int64_t)steps * plan->nstages * per_stage);
+    *launches = (int64_t)fsm::split_parts(plan, batch, steps) * (1 + (int64_t)steps * plan->nstages * per_stage);
   } else if (plan->path == 1 && plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) {
     *launches = steps > 0 ? 3 : 1;  // line kernel, batch means of k = 0, k = 0 fix-up
   } else {
@@ -703,19 +703,33 @@ size_t integrate_workspace_bytes(const FsmPlan* p, int32_t batch, int32_t steps)
 
 namespace fsm {
 // Batches at or above kSplitPoints spectral points run in parts of about kPartPoints points
-// (2 to kMaxParts parts, at most one per sample) on as many streams. Measured on 256^2 x 64
-// (2.1 M points): one sequence 322 us per step, 2 parts 284, 4 parts 270, 8 parts 261.
-constexpr int64_t kSplitPoints = (int64_t)3 << 19;
+// (kMinParts to kMaxParts parts, at most one per sample) on as many streams: one part's passes fill
+// the SMs that another's last wave or its chain of loads leaves idle. us per step, one sequence / 3
+// parts / 4: vorticity 256^2 x 46 179 / 141 / 140, x 20 117 / 111 / 109, 512^2 x 5 161 / 149 / 147,
+// velocity 256^2 x 24 269 / 211 / 205, Burgers 256^2 x 12 112 / 96 / 96, 64^3 x 3 179 / 140; below the
+// line it costs: velocity 256^2 x 8 151 / 158, vorticity 512^2 x 2 110 / 112 (2 parts). At 256^2 x 64: 3 / 4 / 6 /
+// 8 / 12 parts 199.5 / 199.3 / 197.6 / 196.0 / 202.9 with the start of a solve. A solve of few steps below
+// kSplitManyPoints is not worth the parts' events.
+constexpr int64_t kSplitPoints = (int64_t)3 << 17;
+constexpr int64_t kSplitManyPoints = (int64_t)3 << 19;
+constexpr int32_t kSplitSteps = 16;
 constexpr int64_t kPartPoints = (int64_t)1 << 18;
+constexpr int kMinParts = 3;
 constexpr int kMaxParts = 8;
+// Steps between the waits of a part for the part before it, below kMaxParts parts; at kMaxParts every
+// step. Every step / every 4th / never, us per step: 256^2 x 46 in 3 parts 149 / 141, 64^3 x 3 146 / 140,
+// 128^3 x 2 926 / 910 / 912; in 8 parts 128^2 x 300 248 / 252, 256^2 x 128 376 / 378 / 398 (without them the
+// parts drift apart and the last one ends alone).
+constexpr int32_t kRingSteps = 4;
 
-// Number of parts an uncaptured, unprofiled integrate of `batch` samples runs in (1: one sequence).
-int split_parts(const FsmPlan* p, int batch) {
+// Number of parts an uncaptured, unprofiled integrate of `batch` samples over `steps` runs in (1: one sequence).
+int split_parts(const FsmPlan* p, int batch, int steps) {
   if (p->path != 2 && p->path != 4) return 1;
   if (p->nl == FSM_NL_KS && (p->flags & FSM_FLAG_REMOVE_MEAN)) return 1;  // the batch mean couples the samples
-  if (batch < 2 || (int64_t)batch * p->S < kSplitPoints) return 1;
-  int64_t parts = (int64_t)batch * p->S / kPartPoints;
-  parts = parts < 2 ? 2 : (parts > kMaxParts ? kMaxParts : parts);
+  const int64_t points = (int64_t)batch * p->S;
+  if (batch < 2 || points < (steps < kSplitSteps ? kSplitManyPoints : kSplitPoints)) return 1;
+  int64_t parts = points / kPartPoints;
+  parts = parts < kMinParts ? kMinParts : (parts > kMaxParts ? kMaxParts : parts);
   return (int)(parts < batch ? parts : batch);
 }
 }  // namespace fsm
@@ -987,7 +1001,7 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   // which fills the SMs better than one launch sequence of the whole batch.
   // Samples are independent except under the KS batch-wide mean; capture and the profiled
   // (per-launch timed) call keep one sequence.
-  const int NP = (!allow_split || prof || cap != cudaStreamCaptureStatusNone) ? 1 : fsm::split_parts(p, batch);
+  const int NP = (!allow_split || prof || cap != cudaStreamCaptureStatusNone) ? 1 : fsm::split_parts(p, batch, steps);
   const bool split = NP > 1;
   if (!split) {
     PlaneSequence q{p, batch_arrays(p, a, arr, 0, batch), record_slot, steps, st, prof};
@@ -996,8 +1010,9 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
       if ((rc = q.step(k))) return rc;
     return FSM_OK;
   }
-  // The parts are enqueued step by step, each part's step waiting for the previous step of
-  // the part before it (a ring), so that none runs ahead and leaves the others alone at the end.
+  // The parts are enqueued step by step; every `ring` steps each part waits for the part before
+  // it (a ring), so that none runs far ahead and leaves the others alone at the end.
+  const int32_t ring = NP < kMaxParts ? fsm::kRingSteps : 1;
   std::shared_ptr<SplitStreams> streams;
   if ((rc = split_streams(st, &streams))) return rc;
   const cudaStream_t* sub = streams->s;
@@ -1018,9 +1033,10 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   }
   for (int k = 0; k < steps && !rc; ++k) {
     for (int h = 0; h < NP && !rc; ++h) {
-      rc = cuda_check(cudaStreamWaitEvent(sub[h], done[(h + NP - 1) % NP], 0), "step wait");
+      if (k % ring == 0) rc = cuda_check(cudaStreamWaitEvent(sub[h], done[(h + NP - 1) % NP], 0), "step wait");
       if (!rc) rc = q[h].step(k);
     }
+    if ((k + 1) % ring != 0 && k + 1 < steps) continue;
     for (int h = 0; h < NP && !rc; ++h) rc = cuda_check(cudaEventRecord(done[h], sub[h]), "step event");
   }
   for (int h = 0; h < NP && !rc; ++h) rc = cuda_check(cudaStreamWaitEvent(st, done[h], 0), "join wait");

@@ -142,7 +142,7 @@ int launch_plane_row(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_ks_mean(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int launch_pointwise(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 // Parts (streams) an uncaptured integrate of `batch` samples is split into; 1: one sequence.
-int split_parts(const FsmPlan* p, int batch);
+int split_parts(const FsmPlan* p, int batch, int steps);
 
 // The shape of a resident 2D launch (fsm_resident.cu): cluster size, kept / other columns and rows
 // per CTA, product pitch, groups per column, threads and shared memory of a CTA.
