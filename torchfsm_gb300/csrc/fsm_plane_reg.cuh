@@ -434,6 +434,10 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, i
 #pragma unroll
     for (int f = 0; f < CG; ++f) st[f][j] = cscale(st[f][j], m);
   }
+  // The streamfunction's 1 / lap: fast division up to 256 points (within 2 ulp for |lap| below 2^126, far
+  // above any mesh's 2 (pi NX / L)^2; rounded division cost 1% of a step of 256^2 x 64); rounded at 512
+  // points, as those grids always had it.
+  constexpr bool exact = NX == 512;
   // (channel by channel for the Leray projection's groups: the fields of channel f are 2 f, 2 f + 1)
 #pragma unroll
   for (int f = 0; f < CG; ++f) {
@@ -448,8 +452,7 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, i
       float2 x = st[f][j];
       if (KIND == FSM_NL_VORTICITY) {
         const float lap = -(kxv * kxv + gk.ky * gk.ky);
-        // fast division: within 2 ulp for |lap| below 2^126, far above any mesh's 2 (pi NX / L)^2
-        const float il = (lap == 0.f) ? 1.f : __fdividef(1.f, lap);
+        const float il = (lap == 0.f) ? 1.f : exact ? 1.f / lap : __fdividef(1.f, lap);
         x = cscale(x, mf < 2 ? -il : 1.f);
       }
       const float2 ix = cscale(cmuli(x), kxv);
