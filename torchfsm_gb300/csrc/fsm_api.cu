@@ -28,19 +28,9 @@ int cuda_check(cudaError_t e, const char* what) {
   return set_error(code, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-static std::mutex g_attr_mutex;
-static std::map<std::pair<const void*, int>, size_t> g_attr;
-
-bool smem_attr_known(const void* kernel, int device, size_t smem) {
-  std::lock_guard<std::mutex> lock(g_attr_mutex);
-  auto it = g_attr.find({kernel, device});
-  return it != g_attr.end() && it->second >= smem;
-}
-
-void smem_attr_record(const void* kernel, int device, size_t smem) {
-  std::lock_guard<std::mutex> lock(g_attr_mutex);
-  size_t& v = g_attr[{kernel, device}];
-  if (smem > v) v = smem;
+SmemAttributes& smem_attributes() {
+  static SmemAttributes a;
+  return a;
 }
 
 // ---------------------------------------------------------------------------

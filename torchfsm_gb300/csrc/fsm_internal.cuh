@@ -2,6 +2,7 @@
 #pragma once
 
 #include "fsm_common.cuh"
+#include "fsm_smem_attr.h"
 
 namespace fsm {
 
@@ -183,20 +184,17 @@ inline int launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, siz
 // Raise a kernel's dynamic shared-memory limit when it needs more than 48 KB. The
 // attribute is per function and per device; the size set is remembered per
 // (kernel, device) so that repeated launches skip the attribute call.
-bool smem_attr_known(const void* kernel, int device, size_t smem);
-void smem_attr_record(const void* kernel, int device, size_t smem);
+SmemAttributes& smem_attributes();
 
 template <class K>
 inline int prep_smem(K kernel, size_t smem) {
   if (smem <= 48 * 1024) return FSM_OK;
   int dev = 0;
   cudaGetDevice(&dev);
-  const void* key = (const void*)kernel;
-  if (smem_attr_known(key, dev, smem)) return FSM_OK;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute");
-  smem_attr_record(key, dev, smem);
-  return FSM_OK;
+  return smem_attributes().raise((const void*)kernel, dev, smem, [&] {
+    return cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                      "cudaFuncSetAttribute");
+  });
 }
 
 }  // namespace fsm
