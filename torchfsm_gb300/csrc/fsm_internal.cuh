@@ -122,7 +122,8 @@ int launch_line_multi(LineMulti& m, int kind, cudaStream_t st);
 // One launch of the 2D register column (or row) pass over the samples of several plans of square
 // grids (64, 128 or 256 points per axis, Convection or VorticityConvection): entry j runs the pass
 // on a[j].B samples of a[j] (arguments of plane_args, stage and emit set by the caller). gx and
-// cta0 are filled in by the launchers. fast: the SETDRK4 stage launch (stage >= 0).
+// cta0 are filled in by the launchers. A column launch primes every entry (stage -1) or runs a SETDRK4
+// stage of every entry; others are refused.
 constexpr int kPlaneMultiMax = 8;
 struct PlaneMulti {
   StepArgs a[kPlaneMultiMax];
@@ -131,7 +132,7 @@ struct PlaneMulti {
   int32_t cta0[kPlaneMultiMax + 1];
   int32_t count;
 };
-int launch_plane_col_multi(PlaneMulti& m, int kind, bool fast, cudaStream_t st);
+int launch_plane_col_multi(PlaneMulti& m, int kind, cudaStream_t st);
 int launch_plane_row_multi(PlaneMulti& m, int kind, cudaStream_t st);
 // The plane passes' arguments for `batch` samples of `state` advanced by `steps` steps without
 // recording, with the pass arrays in `workspace` laid out as fsm_integrate lays them out (fsm_api.cu).

@@ -23,7 +23,8 @@ constexpr int kept_prefix() {
 
 }  // namespace
 
-template <int KIND, bool FAST>
+// PRIME: the priming launch; else a SETDRK4 stage launch.
+template <int KIND, bool PRIME>
 __device__ __forceinline__ void axis0_multi_body(const PlaneMulti& m) {
   int local = 0;
   const int j = multi_entry(m, &local);
@@ -32,9 +33,9 @@ __device__ __forceinline__ void axis0_multi_body(const PlaneMulti& m) {
   for (int cg = 0; cg < RegKind<KIND, 2>::C / RegKind<KIND, 2>::CG; ++cg) {
     if (cg) __syncthreads();  // the group before is done with the tiles
     switch (m.n[j]) {
-      case 64: axis0_body<64, KIND, 2, FAST>(m.a[j], tile, b, cg); break;
-      case 128: axis0_body<128, KIND, 2, FAST>(m.a[j], tile, b, cg); break;
-      case 256: axis0_body<256, KIND, 2, FAST>(m.a[j], tile, b, cg); break;
+      case 64: axis0_body<64, KIND, 2, !PRIME, -1, PRIME>(m.a[j], tile, b, cg); break;
+      case 128: axis0_body<128, KIND, 2, !PRIME, -1, PRIME>(m.a[j], tile, b, cg); break;
+      case 256: axis0_body<256, KIND, 2, !PRIME, -1, PRIME>(m.a[j], tile, b, cg); break;
     }
   }
 }
@@ -42,12 +43,12 @@ __device__ __forceinline__ void axis0_multi_body(const PlaneMulti& m) {
 // The SETDRK4 stage launches (the hoisted update, two CTAs per SM) and the priming launch.
 template <int KIND>
 __global__ void __launch_bounds__(256, 2) k_axis0_multi2(const __grid_constant__ PlaneMulti m) {
-  axis0_multi_body<KIND, true>(m);
+  axis0_multi_body<KIND, false>(m);
 }
 
 template <int KIND>
 __global__ void __launch_bounds__(256) k_axis0_multi(const __grid_constant__ PlaneMulti m) {
-  axis0_multi_body<KIND, false>(m);
+  axis0_multi_body<KIND, true>(m);
 }
 
 template <int KIND>
@@ -116,12 +117,12 @@ int multi_layout(PlaneMulti& m, bool column, size_t* smem, int* total) {
 }
 
 template <int KIND>
-int launch_col_multi_kind(PlaneMulti& m, bool fast, cudaStream_t st) {
+int launch_col_multi_kind(PlaneMulti& m, bool prime, cudaStream_t st) {
   size_t smem = 0;
   int total = 0;
   int rc = multi_layout<KIND>(m, true, &smem, &total);
   if (rc) return rc;
-  if (fast) {
+  if (!prime) {
     if ((rc = prep_smem(k_axis0_multi2<KIND>, smem))) return rc;
     k_axis0_multi2<KIND><<<total, 256, smem, st>>>(m);
     return cuda_check(cudaGetLastError(), "k_axis0_multi2");
@@ -144,10 +145,16 @@ int launch_row_multi_kind(PlaneMulti& m, cudaStream_t st) {
 
 }  // namespace
 
-int launch_plane_col_multi(PlaneMulti& m, int kind, bool fast, cudaStream_t st) {
+int launch_plane_col_multi(PlaneMulti& m, int kind, cudaStream_t st) {
+  if (m.count < 1 || m.count > kPlaneMultiMax) return set_error(FSM_ERR_INVALID, "plane multi: plan count");
+  // one kernel primes, the other one runs SETDRK4 stages (other schemes need shared memory of their own)
+  const bool prime = m.a[0].stage < 0;
+  for (int j = 0; j < m.count; ++j)
+    if (prime ? m.a[j].stage >= 0 : (m.a[j].stage < 0 || m.a[j].stage > 3 || m.a[j].integ != FSM_SETDRK4))
+      return set_error(FSM_ERR_UNSUPPORTED, "plane multi: priming or SETDRK4 stage launches only");
   switch (kind) {
-    case FSM_NL_CONVECTION: return launch_col_multi_kind<FSM_NL_CONVECTION>(m, fast, st);
-    case FSM_NL_VORTICITY: return launch_col_multi_kind<FSM_NL_VORTICITY>(m, fast, st);
+    case FSM_NL_CONVECTION: return launch_col_multi_kind<FSM_NL_CONVECTION>(m, prime, st);
+    case FSM_NL_VORTICITY: return launch_col_multi_kind<FSM_NL_VORTICITY>(m, prime, st);
   }
   return set_error(FSM_ERR_UNSUPPORTED, "plane multi: Convection or VorticityConvection only");
 }

@@ -327,7 +327,8 @@ __device__ __forceinline__ void axis0_update_any(const StepArgs& a, float2 (&v)[
 //   3. next stage field (mask, 1/N, i kx, streamfunction) -> inverse transform -> mid fields
 // FAST: a SETDRK4 stage launch of a program with channel groups of one channel (the hoisted update,
 // k_axis0_r2); otherwise any scheme, the priming launch included (k_axis0_r). STG: the stage of a FAST launch where the kernel has one of its own
-// (-1: read from the arguments, the multi-plan kernels).
+// (-1: read from the arguments, the multi-plan kernels). PRIME: the priming launch alone (no transform of
+// products, no other update compiled in).
 // The code of a launch is kept small (one stage's update, one copy of the inverse transform).
 // One channel group cg: a CTA of its own per group, so that the channels of a velocity run
 // side by side instead of one after the other (3D Burgers 64^3 x 3: the x pass had 198 CTAs of three
@@ -337,7 +338,7 @@ __device__ __forceinline__ void axis0_update_any(const StepArgs& a, float2 (&v)[
 // field through shared tiles, tables loaded as used): vorticity 256^2 x 64 9.45 -> 8.68 ms per 50
 // steps, 512^2 x 5 6.86 -> 6.37 ms per 40, 3D Burgers 256^3 17.0 -> 14.3 ms per 4, 64^3 x 3 5.62 ->
 // 5.06 ms per 20.
-template <int NX, int KIND, int DIM, bool FAST, int STG = -1>
+template <int NX, int KIND, int DIM, bool FAST, int STG = -1, bool PRIME = false>
 __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, int cg) {
   using Cfg = ColCfg<NX>;
   using K = RegKind<KIND, DIM>;
@@ -359,7 +360,7 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, i
 
   float2 st[CG][E];
   float2 o1[FAST ? E : 1];
-  if (a.stage >= 0) {
+  if (!PRIME && a.stage >= 0) {
 #pragma unroll
     for (int f = 0; f < CG; ++f) {
       const float2* src = a.prod + ((int64_t)b * a.n_prod + cg * CG + f) * a.ms + j0;
@@ -378,7 +379,9 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, i
     __syncthreads();
   }
   if (in) {
-    if constexpr (FAST && STG >= 0) {
+    if constexpr (PRIME) {
+      axis0_update<NX, KIND, DIM, -1, -1>(a, st, b, j0, t, cg, last);
+    } else if constexpr (FAST && STG >= 0) {
       axis0_update_hoisted<NX, KIND, DIM, (STG >= 0 ? STG : 0)>(a, st[0], o1, b, j0, t, cg, last);
     } else if constexpr (FAST) {
       switch (a.stage) {

@@ -450,7 +450,7 @@ int plane_tick(FsmServeGroup* g, int32_t k, int64_t* launched) {
     pm.a[j].stage = -1;
     pm.a[j].emit = 1;
   }
-  if ((rc = fsm::launch_plane_col_multi(pm, g->kind, false, g->st))) return rc;
+  if ((rc = fsm::launch_plane_col_multi(pm, g->kind, g->st))) return rc;
   *launched = 1;
   const int ns = g->m[0]->plan->nstages;
   for (int32_t step = 0; step < k; ++step) {
@@ -460,7 +460,7 @@ int plane_tick(FsmServeGroup* g, int32_t k, int64_t* launched) {
         pm.a[j].stage = st;
         pm.a[j].emit = !(st == ns - 1 && step == k - 1);
       }
-      if ((rc = fsm::launch_plane_col_multi(pm, g->kind, true, g->st))) return rc;
+      if ((rc = fsm::launch_plane_col_multi(pm, g->kind, g->st))) return rc;
       *launched += 2;
     }
   }
