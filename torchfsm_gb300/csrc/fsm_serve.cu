@@ -27,6 +27,13 @@ namespace {
 constexpr int kGraphMaxSteps = 64;
 constexpr size_t kGraphCache = 48;
 
+// A captured tick and the launches that a replay makes.
+struct FsmServeGraph {
+  uint64_t key;
+  cudaGraphExec_t exec;
+  int64_t launches;
+};
+
 }  // namespace
 
 struct FsmServe {
@@ -50,8 +57,8 @@ struct FsmServe {
   int32_t tick_k = 0, tick_n = 0;
   double step_ms = 0.0;  // device time per step and slot, running mean over ticks
   // captured ticks, least recently used first
-  std::list<std::pair<uint64_t, cudaGraphExec_t>> lru;
-  std::unordered_map<uint64_t, std::list<std::pair<uint64_t, cudaGraphExec_t>>::iterator> graphs;
+  std::list<FsmServeGraph> lru;
+  std::unordered_map<uint64_t, std::list<FsmServeGraph>::iterator> graphs;
   std::unordered_set<uint64_t> seen;
   std::vector<int64_t> done_ids;  // completed, not yet reported
   FsmServeGroup* group = nullptr;  // ticked by this group (fsm_serve_group_*), not on its own
@@ -102,7 +109,7 @@ int retire(FsmServe* s, const std::vector<fsm::ServeRequest*>& leaving) {
 }
 
 void drop_graphs(FsmServe* s) {
-  for (auto& e : s->lru) cudaGraphExecDestroy(e.second);
+  for (auto& e : s->lru) cudaGraphExecDestroy(e.exec);
   s->lru.clear();
   s->graphs.clear();
 }
@@ -127,23 +134,27 @@ int advance(FsmServe* s, int32_t n, int32_t k, int64_t* launches) {
         return irc;
       }
       if ((rc = cuda_check(ec, "serve end capture"))) return rc;
-      cudaGraphExec_t ex = nullptr;
-      rc = cuda_check(cudaGraphInstantiate(&ex, g, 0), "serve graph instantiate");
+      FsmServeGraph captured{key, nullptr, 0};
+      size_t nodes = 0;  // every node of a tick is a kernel: no copies, no recording
+      rc = cuda_check(cudaGraphGetNodes(g, nullptr, &nodes), "serve graph nodes");
+      captured.launches = (int64_t)nodes;
+      if (!rc) rc = cuda_check(cudaGraphInstantiate(&captured.exec, g, 0), "serve graph instantiate");
       cudaGraphDestroy(g);
       if (rc) return rc;
-      s->lru.emplace_back(key, ex);
+      s->lru.push_back(captured);
       it = s->graphs.emplace(key, std::prev(s->lru.end())).first;
       while (s->lru.size() > kGraphCache) {
-        s->graphs.erase(s->lru.front().first);
-        cudaGraphExecDestroy(s->lru.front().second);  // freed once a replay in flight completes
+        s->graphs.erase(s->lru.front().key);
+        cudaGraphExecDestroy(s->lru.front().exec);  // freed once a replay in flight completes
         s->lru.pop_front();
       }
     }
     if (it != s->graphs.end()) {
       s->lru.splice(s->lru.end(), s->lru, it->second);
-      if ((rc = cuda_check(cudaGraphLaunch(it->second->second, s->st), "serve graph launch"))) return rc;
+      if ((rc = cuda_check(cudaGraphLaunch(it->second->exec, s->st), "serve graph launch"))) return rc;
       ++s->replays;
-      return fsm_plan_launch_count(s->plan, 0, k, launches);
+      *launches = it->second->launches;
+      return FSM_OK;
     }
     s->seen.insert(key);
   }
