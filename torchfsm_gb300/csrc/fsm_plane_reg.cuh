@@ -437,29 +437,33 @@ __device__ __forceinline__ void axis0_body(const StepArgs& a, int tile, int b, i
 #pragma unroll
     for (int f = 0; f < CG; ++f) st[f][j] = cscale(st[f][j], m);
   }
-  // The streamfunction's 1 / lap: fast division up to 256 points (within 2 ulp for |lap| below 2^126, far
-  // above any mesh's 2 (pi NX / L)^2; rounded division cost 1% of a step of 256^2 x 64); rounded at 512
-  // points, as those grids always had it.
+  // The streamfunction's 1 / lap, once a point: fast division up to 256 points (within 2 ulp for |lap| below
+  // 2^126, far above any mesh's 2 (pi NX / L)^2), rounded at 512 points, as those grids always had it. Once
+  // a field, rounded: vorticity 512^2 x 5 5.21 ms per 40 steps; once a point: 4.76 (4.79 with the fast
+  // division once a field; 256^2 x 64 8.29 -> 7.96 ms per 50).
   constexpr bool exact = NX == 512;
   // (channel by channel for the Leray projection's groups: the fields of channel f are 2 f, 2 f + 1)
 #pragma unroll
   for (int f = 0; f < CG; ++f) {
 #pragma unroll 1
-  for (int mf = f * 2; mf < (CG > 1 ? f * 2 + 2 : K::NMG); ++mf) {
+  for (int i = f * 2; i < (CG > 1 ? f * 2 + 2 : K::NMG); ++i) {
+    // vorticity: 0: psi = -w/lap, 1: i kx psi, 2: w, 3: i kx w, the fields of w first and psi in w's place
+    // then; KS: 0: phi, 1: i kx phi; velocity (per channel): u_c, i kx u_c
+    const int mf = KIND == FSM_NL_VORTICITY ? (i + 2) & 3 : i;
+    if (KIND == FSM_NL_VORTICITY && mf == 0) {
+#pragma unroll
+      for (int j = 0; j < E; ++j) {
+        const float kxv = kxs[t + T * j];
+        const float lap = -(kxv * kxv + gk.ky * gk.ky);
+        const float il = (lap == 0.f) ? 1.f : exact ? 1.f / lap : __fdividef(1.f, lap);
+        st[f][j] = cscale(st[f][j], -il);
+      }
+    }
     float2 v[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-      // vorticity: 0: psi = -w/lap, 1: i kx psi, 2: w, 3: i kx w; KS: 0: phi, 1: i kx phi;
-      // velocity (per channel): u_c, i kx u_c
-      const float kxv = kxs[t + T * j];
-      float2 x = st[f][j];
-      if (KIND == FSM_NL_VORTICITY) {
-        const float lap = -(kxv * kxv + gk.ky * gk.ky);
-        const float il = (lap == 0.f) ? 1.f : exact ? 1.f / lap : __fdividef(1.f, lap);
-        x = cscale(x, mf < 2 ? -il : 1.f);
-      }
-      const float2 ix = cscale(cmuli(x), kxv);
-      v[j] = (mf & 1) ? ix : x;
+      const float2 ix = cscale(cmuli(st[f][j]), kxs[t + T * j]);
+      v[j] = (mf & 1) ? ix : st[f][j];
     }
     col_fft<NX, true>(v, buf, par, twt, t, g);
     const int mout = (KIND == FSM_NL_CONVECTION) ? cg * 2 + mf : mf;
