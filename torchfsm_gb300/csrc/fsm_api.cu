@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "fsm_internal.cuh"
+#include "fsm_split.h"
 
 namespace fsm {
 
@@ -869,6 +870,26 @@ struct PlaneSequence {
   }
 };
 
+// The parts of a split batch as run_parts enqueues them.
+struct SplitRun {
+  cudaStream_t st = nullptr;
+  const cudaStream_t* sub = nullptr;
+  SplitEvents ev;
+  PlaneSequence q[kMaxParts];
+
+  int fork() { return cuda_check(cudaEventRecord(ev.fork, st), "fork"); }
+  int begin(int h) { return cuda_check(cudaStreamWaitEvent(sub[h], ev.fork, 0), "fork wait"); }
+  int prime(int h) { return q[h].prime(); }
+  int step(int h, int k) { return q[h].step(k); }
+  int record(int h) { return cuda_check(cudaEventRecord(ev.done[h], sub[h]), "step event"); }
+  int wait(int h, int g) { return cuda_check(cudaStreamWaitEvent(sub[h], ev.done[g], 0), "step wait"); }
+  int join(int h) { return cuda_check(cudaStreamWaitEvent(st, ev.done[h], 0), "join wait"); }
+  void finish(int h) {  // without a message of its own: the caller gets the first failure's
+    if (cudaEventRecord(ev.done[h], sub[h]) != cudaSuccess || cudaStreamWaitEvent(st, ev.done[h], 0) != cudaSuccess)
+      cudaStreamSynchronize(sub[h]);
+  }
+};
+
 }  // namespace
 
 namespace fsm {
@@ -1000,39 +1021,19 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
       if ((rc = q.step(k))) return rc;
     return FSM_OK;
   }
-  // The parts are enqueued step by step; every `ring` steps each part waits for the part before
-  // it (a ring), so that none runs far ahead and leaves the others alone at the end.
   const int32_t ring = NP < kMaxParts ? fsm::kRingSteps : 1;
   std::shared_ptr<SplitStreams> streams;
   if ((rc = split_streams(st, &streams))) return rc;
-  const cudaStream_t* sub = streams->s;
-  SplitEvents ev;
-  if ((rc = ev.create(NP))) return rc;
-  const cudaEvent_t fork = ev.fork;
-  const cudaEvent_t* done = ev.done;
-  PlaneSequence q[kMaxParts];
+  SplitRun run;
+  if ((rc = run.ev.create(NP))) return rc;
+  run.st = st;
+  run.sub = streams->s;
   for (int h = 0; h < NP; ++h) {
     const int b0 = (int)((int64_t)batch * h / NP), b1 = (int)((int64_t)batch * (h + 1) / NP);
-    q[h] = PlaneSequence{p, batch_arrays(p, a, arr, b0, b1 - b0), record_slot, steps, sub[h], nullptr};
+    run.q[h] = PlaneSequence{p, batch_arrays(p, a, arr, b0, b1 - b0), record_slot, steps, run.sub[h], nullptr};
   }
-  rc = cuda_check(cudaEventRecord(fork, st), "fork");
-  for (int h = 0; h < NP && !rc; ++h) {
-    rc = cuda_check(cudaStreamWaitEvent(sub[h], fork, 0), "fork wait");
-    if (!rc) rc = q[h].prime();
-    if (!rc) rc = cuda_check(cudaEventRecord(done[h], sub[h]), "step event");
-  }
-  for (int k = 0; k < steps && !rc; ++k) {
-    for (int h = 0; h < NP && !rc; ++h) {
-      if (k % ring == 0) rc = cuda_check(cudaStreamWaitEvent(sub[h], done[(h + NP - 1) % NP], 0), "step wait");
-      if (!rc) rc = q[h].step(k);
-    }
-    if ((k + 1) % ring != 0 && k + 1 < steps) continue;
-    for (int h = 0; h < NP && !rc; ++h) rc = cuda_check(cudaEventRecord(done[h], sub[h]), "step event");
-  }
-  for (int h = 0; h < NP && !rc; ++h) rc = cuda_check(cudaStreamWaitEvent(st, done[h], 0), "join wait");
-  return rc;
+  return run_parts(run, NP, steps, ring);
 }
-
 
 }  // namespace
 
