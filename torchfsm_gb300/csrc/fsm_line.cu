@@ -58,6 +58,13 @@ __device__ __forceinline__ void line_body(const StepArgs& a, int b, int t, int i
   constexpr int M = E / 2 + 1;  // modes t + T j, j < M (the last one, N/2, is thread 0's)
   // the buffers alternate over the exchanges of a stage: two transforms and the conjugate modes
   constexpr int XF = line_exchanges<N>();
+  // A transform of up to 64 points takes T < 32 lanes with M modes each. The schemes dispatched at run time
+  // (REGS false) spread the modes over the whole warp for their update, through the exchange buffers: M updates one
+  // after the other cost more than the exchange (RK4 of one sample, 40 steps, us: 16 points 185 -> 115, 32: 201 -> 134, 64:
+  // 214 -> 166).
+  constexpr bool SPREAD = !REGS && T < 32;
+  constexpr int MW = (H + 31) / 32;  // modes of a lane then
+  const int lane = threadIdx.x & 31;
   float2* u = reg + 2 * Cfg::NB;
   float2* acc = u + H;  // running sums: acc, q (Runge-Kutta: n_aux arrays H apart)
   float2* q = acc + H;
@@ -97,6 +104,15 @@ __device__ __forceinline__ void line_body(const StepArgs& a, int b, int t, int i
     }
   };
 
+  float skx[SPREAD ? MW : 1], smask[SPREAD ? MW : 1];
+  if constexpr (SPREAD) {
+#pragma unroll
+    for (int r = 0; r < MW; ++r) {
+      const int k = min(lane + 32 * r, N / 2);
+      skx[r] = a.kx[k];
+      smask[r] = (float)a.keepx[k] * a.scale;
+    }
+  }
   float2 x[M];
   if (on) {
 #pragma unroll
@@ -141,6 +157,37 @@ __device__ __forceinline__ void line_body(const StepArgs& a, int b, int t, int i
       const int slot = (last && a.slots) ? a.slots[step + 1] : -1;
       // k = 0 of the product, for the batch-mean fix-up (k_line_dc_fixup)
       if (dc) a.dc[((int64_t)step * ns + s) * a.B + b] = v[0];
+      if constexpr (SPREAD) {
+        float2* ex = reg + par * Cfg::NB;
+        float2* zx = reg + (par ^ 1) * Cfg::NB;
+        if (on) {
+#pragma unroll
+          for (int j = 0; j < M; ++j) {
+            if (j == M - 1 && t != 0) break;
+            ex[line_pad(t + T * j)] = v[j];
+          }
+        }
+        line_sync<N>(id);
+#pragma unroll
+        for (int r = 0; r < MW; ++r) {
+          const int k = lane + 32 * r;
+          if (k < H) {
+            float2 nv = cscale(ex[line_pad(k)], a.coef);
+            if (src) nv = cadd(nv, src[k]);
+            const float2 xk = etd_stage(a.integ, s, nv, u + k, acc + k, q + k, tab + k, a.ts, H);
+            if (slot >= 0 && active) a.traj[((int64_t)b * a.n_frames + slot) * H + k] = xk;
+            float2 mir;
+            zx[line_pad(k)] = line_build<N, KIND>(k, xk, smask[r], skx[r], &mir);
+            if (k > 0 && k < N / 2) zx[line_pad(N - k)] = mir;
+          }
+        }
+        line_sync<N>(id);
+        if (on) {
+#pragma unroll
+          for (int j = 0; j < E; ++j) v[j] = zx[line_pad(t + T * j)];
+        }
+        continue;
+      }
       if (on) {
 #pragma unroll
         for (int j = 0; j < M; ++j) {
