@@ -618,13 +618,14 @@ int fsm_plan_workspace_bytes(const FsmPlan* plan, int32_t batch, int32_t steps, 
 
 int fsm_plan_launch_count(const FsmPlan* plan, int32_t batch, int32_t steps, int64_t* launches) {
   if (!plan || !launches || steps < 0 || batch < 0) return set_error(FSM_ERR_INVALID, "launch_count arguments");
+  const int parts = fsm::split_parts(plan, batch, steps);
   fsm::ResConfig res;
-  if (fsm::resident_config(plan, batch, &res)) {
+  if (fsm::resident_config(plan, batch, parts, &res)) {
     *launches = steps > 0 ? (steps + kResidentSteps - 1) / kResidentSteps : 1;
   } else if (plan->path == 2 || plan->path == 4) {
     const int64_t per_stage = (plan->path == 4 && !fsm::volume_plane_applies(plan) ? 4 : 2) +
                               ((plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) ? 1 : 0);
-    *launches = (int64_t)fsm::split_parts(plan, batch, steps) * (1 + (int64_t)steps * plan->nstages * per_stage);
+    *launches = (int64_t)parts * (1 + (int64_t)steps * plan->nstages * per_stage);
   } else if (plan->path == 1 && plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) {
     *launches = steps > 0 ? 3 : 1;  // line kernel, batch means of k = 0, k = 0 fix-up
   } else {
@@ -971,9 +972,10 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   if ((rc = cuda_check(cudaStreamIsCapturing(st, &cap), "stream capture query"))) return rc;
   // The resident 2D kernel reads the slots from the device too: a captured recording (which the
   // passes take) stays on the passes.
+  const int NP = (!allow_split || prof || cap != cudaStreamCaptureStatusNone) ? 1 : fsm::split_parts(p, batch, steps);
   ResConfig res;
   const bool resident =
-      !prof && !(record_slot && cap != cudaStreamCaptureStatusNone) && resident_config(p, batch, &res);
+      !prof && !(record_slot && cap != cudaStreamCaptureStatusNone) && resident_config(p, batch, NP, &res);
   if (record_slot && (p->path == 1 || p->path == 3 || resident)) {
     if (cap != cudaStreamCaptureStatusNone)
       return set_error(FSM_ERR_INVALID, "integrate: recording is not supported while the stream is being captured");
@@ -1012,9 +1014,7 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   // which fills the SMs better than one launch sequence of the whole batch.
   // Samples are independent except under the KS batch-wide mean; capture and the profiled
   // (per-launch timed) call keep one sequence.
-  const int NP = (!allow_split || prof || cap != cudaStreamCaptureStatusNone) ? 1 : fsm::split_parts(p, batch, steps);
-  const bool split = NP > 1;
-  if (!split) {
+  if (NP == 1) {
     PlaneSequence q{p, batch_arrays(p, a, arr, 0, batch), record_slot, steps, st, prof};
     if ((rc = q.prime())) return rc;
     for (int k = 0; k < steps; ++k)

@@ -153,8 +153,9 @@ struct ResConfig {
   bool tables;
   size_t smem;
 };
-// Whether a whole integrate of `batch` samples runs in the resident 2D kernel, and in which shape.
-bool resident_config(const FsmPlan* p, int batch, ResConfig* out);
+// Whether a whole integrate of `batch` samples runs in the resident 2D kernel, and in which shape; `parts`:
+// what the passes would run in.
+bool resident_config(const FsmPlan* p, int batch, int parts, ResConfig* out);
 // a.steps steps of a.B samples in one launch, frames at a.slots (device) when given.
 int launch_resident(const FsmPlan* p, const ResConfig& c, const StepArgs& a, cudaStream_t st);
 
