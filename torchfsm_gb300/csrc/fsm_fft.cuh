@@ -17,6 +17,11 @@ namespace fsm {
 // sums, and the kernels are bound by instruction issue or by the latency of one warp's chain. Each
 // component rounds as a scalar sum does. Measured: resident 2D kernel 128^2 x 16 (convection)
 // 35.2 -> 33.3 us per step, 128 x 256 (Leray) 91 -> 81; 3D Burgers 256^3 19.9 -> 19.3 ms per 4 steps.
+// nvcc 13.0.88 was seen to compile packed sums wrong: a vorticity row pass with its two rows in a rolled
+// loop, at the 128-register cap, gave wrong products, the same at every run, with a CTA barrier in place of the
+// warp's and with the compiler's own packed intrinsics alike, and right ones with scalar sums or without the cap.
+// Every kernel at the cap is therefore held against the oracle (tests/test_gpu_long_axes.py); the
+// library's results with scalar sums in place of these are the same bit for bit (2264 calls over all sizes and terms).
 __device__ __forceinline__ unsigned long long pack2(float2 a) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
