@@ -155,8 +155,8 @@ int fsm_plan_workspace_bytes(const FsmPlan* plan, int32_t batch, int32_t steps, 
 
 /* Number of kernel launches fsm_integrate makes for `batch` samples and `steps` steps outside
  * stream capture (large batches run in parts, each with its own launches; 2D SETDRK4 solves
- * on the resident kernel make one launch per 2048 steps); batch 0 counts one launch sequence
- * of passes. */
+ * on the resident kernel make one launch per 2048 steps, per 256 where the batch fills the
+ * device); batch 0 counts one launch sequence of passes. */
 int fsm_plan_launch_count(const FsmPlan* plan, int32_t batch, int32_t steps, int64_t* launches);
 
 /* Advance `state` (half spectra, [batch][C][S] complex64, in place) by `steps`

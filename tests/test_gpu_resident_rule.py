@@ -21,3 +21,21 @@ def test_line_between_resident_kernel_and_parts(build, channels, batch, steps, r
     plan.integrate_half(a, steps)
     _passes(plan, b, steps)
     assert torch.equal(torch.view_as_real(a), torch.view_as_real(b))
+
+
+@pytest.mark.parametrize("batch,launches", [(8, 1), (2000, 2)])
+def test_a_full_device_returns_sooner(batch, launches):
+    """A batch that fills the device advances at most 256 steps a launch, others 2048; frames on either side of
+    the boundary."""
+    plan, sp, u, _ = _setup(VORT, (32, 32), batch, 1, 1e-3)
+    assert plan.launch_count(256, batch) == 1 and plan.launch_count(258, batch) == launches
+    a = sp.to_half(u).contiguous()
+    b, frame = a.clone(), a.clone()
+    traj = torch.empty((batch, 3) + tuple(a.shape[1:]), dtype=a.dtype, device=a.device)
+    plan.integrate_half(a, 258, slots=[-1] * 255 + [0, 1, -1, 2], traj=traj)
+    _passes(plan, b, 258)
+    assert torch.equal(a, b) and torch.equal(traj[:, 2], a)
+    for i, steps in enumerate((255, 256)):
+        c = frame.clone()
+        _passes(plan, c, steps)
+        assert torch.equal(traj[:, i], c)

@@ -284,9 +284,6 @@ static int phi_exact(const FsmPlan* p) {
   return bound < 1e-10 ? 1 : 0;
 }
 
-// Steps of one launch of the resident 2D kernel: long runs return to the stream now and then.
-constexpr int32_t kResidentSteps = 2048;
-
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static void free_plan(FsmPlan* p) {
@@ -621,7 +618,7 @@ int fsm_plan_launch_count(const FsmPlan* plan, int32_t batch, int32_t steps, int
   const int parts = fsm::split_parts(plan, batch, steps);
   fsm::ResConfig res;
   if (fsm::resident_config(plan, batch, parts, &res)) {
-    *launches = steps > 0 ? (steps + kResidentSteps - 1) / kResidentSteps : 1;
+    *launches = steps > 0 ? (steps + res.steps - 1) / res.steps : 1;
   } else if (plan->path == 2 || plan->path == 4) {
     const int64_t per_stage = (plan->path == 4 && !fsm::volume_plane_applies(plan) ? 4 : 2) +
                               ((plan->nl == FSM_NL_KS && (plan->flags & FSM_FLAG_REMOVE_MEAN)) ? 1 : 0);
@@ -995,10 +992,10 @@ int integrate_impl(const FsmPlan* p, int32_t batch, void* state, int32_t steps, 
   if (p->path == 1) return timed(prof, kProfOther, [&] { return launch_line(p, a, st); });
 
   if (resident) {
-    // at most kResidentSteps steps a launch (the next one primes from the state it left)
+    // at most res.steps steps a launch (the next one primes from the state it left)
     int32_t done = 0;
     do {
-      a.steps = steps - done < kResidentSteps ? steps - done : kResidentSteps;
+      a.steps = steps - done < res.steps ? steps - done : res.steps;
       if ((rc = launch_resident(p, res, a, st))) return rc;
       done += a.steps;
       if (a.slots) a.slots += a.steps;

@@ -147,9 +147,9 @@ int launch_pointwise(const FsmPlan* p, const StepArgs& a, cudaStream_t st);
 int split_parts(const FsmPlan* p, int batch, int steps);
 
 // The shape of a resident 2D launch (fsm_resident.cu): cluster size, kept / other columns and rows
-// per CTA, product pitch, groups per column, threads and shared memory of a CTA.
+// per CTA, product pitch, groups per column, threads and shared memory of a CTA; steps of a launch at most.
 struct ResConfig {
-  int cl, ka, kb, pc, fs, rpc, threads;
+  int cl, ka, kb, pc, fs, rpc, threads, steps;
   bool tables;
   size_t smem;
 };

@@ -14,6 +14,12 @@ namespace {
 
 constexpr size_t kSmemMax = 227 * 1024;   // per CTA
 constexpr size_t kSmemHalf = 114 * 1024;  // above this one CTA fits per SM
+// Steps of one launch: long runs return to the stream now and then. A batch that fills the device returns
+// sooner, so that a stream of higher priority finds SMs after some milliseconds (2048 steps of 64^2 x 1000
+// hold them for 0.1 s at a time). A launch loads and stores its samples' state and tables: 64^2 x 1000 183.9 -> 184.1
+// us per step, Burgers 128^2 x 30 59.5 -> 59.8.
+constexpr int kResidentSteps = 2048;
+constexpr int kResidentStepsFull = 256;
 
 ResKernel kernel_of(const FsmPlan* p) {
   switch (p->nl) {
@@ -119,6 +125,7 @@ bool resident_config(const FsmPlan* p, int batch, int parts, ResConfig* out) {
     const double est = waves * (1.0 + work / cl) * (1.0 + 0.3 * (shared - 1));
     if (best == 0.0 || est < best) {
       best = est;
+      c.steps = batch < cap ? kResidentSteps : kResidentStepsFull;
       *out = c;
     }
   }
