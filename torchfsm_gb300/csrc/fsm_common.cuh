@@ -336,7 +336,8 @@ struct FsmPlan {
   // 2D and 3D passes: the leading last-axis columns of the stage fields that the passes exchange.
   // Below h when the dealias mask keeps the prefix of n/3 + 1 columns (the 2/3 rule): the fields
   // beyond it are zero, so they are neither stored nor loaded (3D: nor the kept columns of middle-axis
-  // modes that the mask drops).
+  // modes that the mask drops). A value that is not finite in a mode that is skipped so stays in its mode;
+  // where mask times spectrum is formed it spreads (0 x inf) to all of them. Every physical value is lost either way.
   int hk = 0;
   // Row pitch (complex entries) and field stride of the stage fields and products (workspace
   // arrays exchanged between the passes). 2D register passes: n1/2 + 1 rounded up to even, so that
