@@ -359,9 +359,9 @@ AdjLayout adj_layout(const FsmPlan* p, int32_t batch) {
     o += a256(nb * tr * sizeof(float));
   }
   L.Q = o;
-  o += a256(nb * tr * sizeof(float));
+  if (p->ndim != 2) o += a256(nb * tr * sizeof(float));  // (2D: the row kernel keeps these in registers)
   L.nbp = o;
-  o += a256(tr * sizeof(float));
+  if (p->ndim != 2) o += a256(tr * sizeof(float));
   L.F = o;
   o += a256(nb * th * sizeof(float2));
   for (int i = 0; i < 11; ++i) {

@@ -450,8 +450,8 @@ int fsm_plan_create(const FsmMeshDesc* mesh, const FsmProgramDesc* prog, double 
   std::vector<uint8_t> tile_zero;
   {
     const int n0 = mesh->n[0];
-    const int w = n0 == 512 ? 8 : n0 == 256 ? 16 : (n0 == 128 || n0 == 64) ? 32 : (n0 == 32 || n0 == 16) ? 64 : 0;
-    if (w && (path == 2 || path == 4)) {
+    const int w = n0 == 512 ? 8 : n0 == 256 ? 16 : n0 >= 64 ? 32 : 64;  // columns of a CTA (ColCfg)
+    if (path == 2 || path == 4) {
       const int h = mesh->n[nd - 1] / 2 + 1;
       const int64_t inner = p->S / n0;
       auto kept = [&](int64_t j) {
@@ -468,13 +468,12 @@ int fsm_plan_create(const FsmMeshDesc* mesh, const FsmProgramDesc* prog, double 
   }
   p->hk = p->h;
   if (path == 2) {
-    const int n0 = mesh->n[0], n1 = mesh->n[1];
-    const bool reg = is_pow2(n0) && n0 >= 16 && n0 <= 512 && is_pow2(n1) && n1 >= 16 && n1 <= 512;
+    const int n1 = mesh->n[1];
     int pre = 0;
     while (pre < p->h && keep[p->koff[1] + pre]) ++pre;
     bool prefix = true;
     for (int j = pre; j < p->h; ++j) prefix = prefix && !keep[p->koff[1] + j];
-    if (reg && prefix && pre == n1 / 3 + 1) p->hk = pre;
+    if (prefix && pre == n1 / 3 + 1) p->hk = pre;
   }
   if (path == 4) {
     // 3D: the stage fields' kept last-axis prefix, when the mask keeps n2/3 + 1 columns
@@ -486,10 +485,7 @@ int fsm_plan_create(const FsmMeshDesc* mesh, const FsmProgramDesc* prog, double 
     if (prefix && pre == n2 / 3 + 1) p->hk = pre;
   }
   p->wp = p->S / mesh->n[0];
-  if (path == 2) {
-    const int n0 = mesh->n[0], n1 = mesh->n[1];
-    if (is_pow2(n0) && n0 >= 16 && n0 <= 512 && is_pow2(n1) && n1 >= 16 && n1 <= 512) p->wp = (p->h + 1) & ~1;
-  }
+  if (path == 2) p->wp = (p->h + 1) & ~1;
   p->ms = (int64_t)mesh->n[0] * p->wp;
   std::vector<float2> tw(kTwiddleMax);
   for (int k = 0; k < kTwiddleMax; ++k) {
