@@ -9,12 +9,13 @@ from test_gpu_resident import BURG, NSVEL, VORT, _passes, _setup
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("build,channels,batch,steps,resident", [
-    (VORT, 1, 80, 16, True), (VORT, 1, 200, 12, False), (VORT, 1, 128, 16, False),
-    (VORT, 1, 128, 12, True),  # too few steps for parts
-    (BURG, 2, 64, 16, True), (BURG, 2, 100, 16, False), (NSVEL, 2, 100, 16, True)])
-def test_line_between_resident_kernel_and_parts(build, channels, batch, steps, resident):
-    plan, sp, u, _ = _setup(build, (128, 128), batch, channels, 2e-3)
+@pytest.mark.parametrize("build,channels,shape,batch,steps,resident", [
+    (VORT, 1, (128, 128), 80, 16, True), (VORT, 1, (128, 128), 200, 12, False), (VORT, 1, (128, 128), 128, 16, False),
+    (VORT, 1, (128, 128), 128, 12, True),  # too few steps for parts
+    (BURG, 2, (128, 128), 64, 16, True), (BURG, 2, (128, 128), 100, 16, False), (NSVEL, 2, (128, 128), 100, 16, True),
+    (BURG, 2, (128, 256), 24, 16, True), (BURG, 2, (128, 256), 32, 16, False), (NSVEL, 2, (128, 256), 32, 16, True)])
+def test_line_between_resident_kernel_and_parts(build, channels, shape, batch, steps, resident):
+    plan, sp, u, _ = _setup(build, shape, batch, channels, 1e-3)
     assert (plan.launch_count(steps, batch) == 1) == resident
     a = sp.to_half(u).contiguous()
     b = a.clone()

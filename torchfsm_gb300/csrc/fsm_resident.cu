@@ -82,10 +82,11 @@ int active_clusters(const ResKernel& k, const ResConfig& c, size_t smem) {
 // Against the passes (resident / passes): 64^2 vorticity 1 sample 12.2 / 66, 150: 27 / 83, 1000: 185 /
 // 275; 128^2 16: 30 / 108, 128: 152 / 191, 256: 298 / 254; 256^2 7: 39 / 97, 14: 76 / 105, 24: 150 / 134;
 // 128x256 velocity 9: 49 / 170. Above 8192 points the passes win once est x points exceeds 190e3, and sooner
-// where the batch runs in parts (`parts` above 1: medium batches of 16 steps or more, large ones): vorticity
-// 128^2 x 80 (est 4.9) 98 / 102, x 100 (5.4) 117 / 115, x 200 (10.8) 231 / 154; Burgers 128^2 x 80 (4.9)
-// 120 / 121, x 100 (6.6) 158 / 134; 64x256 x 64 (4.6) 93 / 84, x 100 (6.6) 139 / 106. The Leray projection's passes
-// carry both channels in one chain: 128^2 x 100 (6.6) takes 1.2 times as long in parts as here.
+// where the batch runs in parts (`parts` above 1: medium batches of 16 steps or more, large ones), resident /
+// parts: vorticity 128^2 x 80 (est 4.9) 105 / 105, x 100 (5.4) 117 / 111, x 200 (10.8) 231 / 154; Burgers 128^2 x 80
+// (4.9) 119 / 120, x 100 (6.6) 158 / 133; at 32768 points sooner still: 128x256 x 24 (2.9) 80 / 84, x 32 (4.4)
+// 117 / 96, vorticity 256x128 x 24 (2.9) 71 / 83, x 32 (4.4) 104 / 98. The Leray projection's passes carry both
+// channels in one chain: 128^2 x 100 (6.6) takes 1.2 times as long in parts as here.
 bool resident_config(const FsmPlan* p, int batch, int parts, ResConfig* out) {
   const int nx = p->n[0], ny = p->n[1], h = p->h, hk = p->hk;
   if (p->path != 2 || p->integ != FSM_SETDRK4 || batch < 1 || hk != ny / 3 + 1) return false;
@@ -131,7 +132,8 @@ bool resident_config(const FsmPlan* p, int batch, int parts, ResConfig* out) {
   }
   const double points = (double)nx * ny;
   const bool parted = parts > 1 && p->nl != FSM_NL_LERAY;
-  return best > 0.0 && (points <= 8192.0 || (best * points <= 190e3 && !(parted && best > 5.0)));
+  const double line = points > 16384.0 ? 4.2 : 5.0;
+  return best > 0.0 && (points <= 8192.0 || (best * points <= 190e3 && !(parted && best > line)));
 }
 
 int launch_resident(const FsmPlan* p, const ResConfig& c, const StepArgs& a, cudaStream_t st) {
