@@ -689,11 +689,11 @@ size_t integrate_workspace_bytes(const FsmPlan* p, int32_t batch, int32_t steps)
 namespace fsm {
 // Batches at or above kSplitPoints spectral points run in parts of about kPartPoints points
 // (kMinParts to kMaxParts parts, at most one per sample) on as many streams: one part's passes fill
-// the SMs that another's last wave or its chain of loads leaves idle. us per step, one sequence / 3
-// parts / 4: vorticity 256^2 x 46 179 / 141 / 140, x 20 117 / 111 / 109, 512^2 x 5 161 / 149 / 147,
-// velocity 256^2 x 24 269 / 211 / 205, Burgers 256^2 x 12 112 / 96 / 96, 64^3 x 3 179 / 140; below the
-// line it costs: velocity 256^2 x 8 151 / 158, vorticity 512^2 x 2 110 / 112 (2 parts). At 256^2 x 64: 3 / 4 / 6 /
-// 8 / 12 parts 199.5 / 199.3 / 197.6 / 196.0 / 202.9 with the start of a solve. A solve of few steps below
+// the SMs that another's last wave or its chain of loads leaves idle. us per step beyond the start of a
+// solve, one sequence / in parts (their number): vorticity 256^2 x 46 159 / 119 (5), x 20 100 / 94 (3), 512^2 x 5
+// 129 / 117 (3), velocity 256^2 x 24 244 / 188 (3), Burgers 256^2 x 12 99 / 84 (3), 64^3 x 3 145 / 105 (3), 128^3 x 2
+// 912 / 793 (2); below the line it costs for some: velocity 256^2 x 8 128 / 134, vorticity 512^2 x 2 80.4 / 82.5. Vorticity
+// 256^2 x 64: 201 in one sequence, in 4 / 6 / 8 / 12 parts 160 / 159 / 158 / 165. A solve of few steps below
 // kSplitManyPoints is not worth the parts' events.
 constexpr int64_t kSplitPoints = (int64_t)3 << 17;
 constexpr int64_t kSplitManyPoints = (int64_t)3 << 19;
@@ -702,9 +702,9 @@ constexpr int64_t kPartPoints = (int64_t)1 << 18;
 constexpr int kMinParts = 3;
 constexpr int kMaxParts = 8;
 // Steps between the waits of a part for the part before it, below kMaxParts parts; at kMaxParts every
-// step. Every step / every 4th / never, us per step: 256^2 x 46 in 3 parts 149 / 141, 64^3 x 3 146 / 140,
-// 128^3 x 2 926 / 910 / 912; in 8 parts 128^2 x 300 248 / 252, 256^2 x 128 376 / 378 / 398 (without them the
-// parts drift apart and the last one ends alone).
+// step. Every step / every 4th / never, us per step: vorticity 256^2 x 46 in 5 parts 125 / 119 / 118, 64^3 x 3
+// 111 / 105 / 104, 128^3 x 2 803 / 793 / 790; in 8 parts vorticity 128^2 x 300 221 / 222 / 231, 256^2 x 128 329 / 330 / 351
+// (without them the parts drift apart and the last one ends alone).
 constexpr int32_t kRingSteps = 4;
 
 // Number of parts an uncaptured, unprofiled integrate of `batch` samples over `steps` runs in (1: one sequence).
